@@ -15,7 +15,8 @@ OUT = os.path.join(HERE, "build")
 ROOT = os.path.dirname(HERE)
 NVCC = os.environ.get("NVCC", "nvcc")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-CU_SOURCES = ["dsgl_window.cu", "dsgl_plain.cu", "dsgl_aux.cu", "dsgl_adjoint.cu", "dsgl_noalloc.cu",
+CU_SOURCES = ["dsgl_window.cu", "dsgl_team.cu", "dsgl_team_f32_k5.cu", "dsgl_team_f32_k10.cu", "dsgl_team_bf16_k5.cu",
+              "dsgl_team_bf16_k10.cu", "dsgl_plain.cu", "dsgl_aux.cu", "dsgl_adjoint.cu", "dsgl_noalloc.cu",
               "dsgl_ingest.cu", "dsgl_eval.cu", "dsgl_walk.cu"]
 CPP_SOURCES = ["sgns_host.cpp"]
 LIB = os.path.join(OUT, "libsgns.so")

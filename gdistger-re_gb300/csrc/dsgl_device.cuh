@@ -373,197 +373,161 @@ __device__ __forceinline__ void forward_gradient(int I, int first, int O, int d,
   __syncwarp();
 }
 
-// Forward of the persistent engine: the same gradient, with each dot product summed as
-// eight independent sequential partial sums -- the even and the odd k of each quarter of
-// [0, d), each pair advanced by one FFMA2 on {o[k], o[k+1]} x {x[k], x[k+1]} -- combined
-// as s_m = even_m + odd_m, f = (s_0 + s_1) + (s_2 + s_3) when d % 16 == 0; when not,
-// [0, d) is one range and f = even + odd.  The oracle's window policy uses the same
-// order.  out_rows: normal layout, stride DP.
-// One round over inputs j0..j0+nj-1 with L lanes per input (NQ * L == 4 quarters per
-// input, or kWhole: the whole range, one lane per input).  Lane pairs (L == 2) each hold
-// (s0 + s1) or (s2 + s3) and add the other's with a shuffle (a + b == b + a bit for bit).
-template <int NQ, int L, bool kWhole, int OM, class InPtr>
-__device__ __forceinline__ void forward_round(int j0, int nj, int first, int O, int q4, InPtr in_ptr,
-                                              const float* out_rows, int DP, const int* out_meta,
-                                              const float* exp_table, float alpha, float2* corrP,
-                                              bool want_loss, float& loss) {
-  typedef StepShape<OM> SS;
-  const int lane = lane_id();
-  const int jl = lane / L, sub = lane % L;
-  const int j = j0 + jl;
-  const bool active = jl < nj;
-  const float4* x = reinterpret_cast<const float4*>(in_ptr(active ? j : j0));
-  const int m0 = sub * NQ;
-  float2 f[OM][NQ];
-#pragma unroll
-  for (int i = 0; i < OM; i++)
-#pragma unroll
-    for (int m = 0; m < NQ; m++) f[i][m] = make_float2(0.f, 0.f);
-  for (int k4 = 0; k4 < q4; k4++) {
-    float4 xv[NQ];
-#pragma unroll
-    for (int m = 0; m < NQ; m++) xv[m] = x[(m0 + m) * q4 + k4];
-#pragma unroll
-    for (int i = 0; i < OM; i++) {
-      const float4* orow = reinterpret_cast<const float4*>(out_rows + (size_t)i * DP);
-#pragma unroll
-      for (int m = 0; m < NQ; m++) {
-        const float4 o = orow[(m0 + m) * q4 + k4];
-        f[i][m] = ffma2(make_float2(o.x, o.y), make_float2(xv[m].x, xv[m].y), f[i][m]);
-        f[i][m] = ffma2(make_float2(o.z, o.w), make_float2(xv[m].z, xv[m].w), f[i][m]);
-      }
-    }
-  }
-  float fv[OM];
-#pragma unroll
-  for (int i = 0; i < OM; i++) {
-    if (kWhole) {
-      fv[i] = __fadd_rn(f[i][0].x, f[i][0].y);
-    } else if (NQ == 4) {
-      const float s0 = __fadd_rn(f[i][0].x, f[i][0].y), s1 = __fadd_rn(f[i][1 % NQ].x, f[i][1 % NQ].y);
-      const float s2 = __fadd_rn(f[i][2 % NQ].x, f[i][2 % NQ].y), s3 = __fadd_rn(f[i][3 % NQ].x, f[i][3 % NQ].y);
-      fv[i] = __fadd_rn(__fadd_rn(s0, s1), __fadd_rn(s2, s3));
-    } else {
-      const float a = __fadd_rn(__fadd_rn(f[i][0].x, f[i][0].y), __fadd_rn(f[i][1 % NQ].x, f[i][1 % NQ].y));
-      fv[i] = __fadd_rn(a, __shfl_xor_sync(kFull, a, 1));
-    }
-  }
-  if (active && sub == 0) {
-#pragma unroll
-    for (int i = 0; i < OM; i++) {
-      if (i < O) {
-        const float fi = fv[i];
-        const int label = j < first ? (i == 0) : (i == 1);  // outputs t1, t2, negatives
-        float g;
-        if (fi > (float)kMaxExp) {
-          g = __fmul_rn((float)(label - 1), alpha);
-        } else if (fi < -(float)kMaxExp) {
-          g = __fmul_rn((float)label, alpha);
-        } else {
-          const int idx = __float2int_rz(__fmul_rn(__fadd_rn(fi, (float)kMaxExp), (float)kTableScale));
-          g = __fmul_rn(__fsub_rn((float)label, exp_table[idx]), alpha);
-        }
-        const float gm = __fmul_rn(g, (float)out_meta[i]);
-        corrP[j * SS::CS + i] = make_float2(gm, gm);
-        if (want_loss) {
-          const float z = label ? -fi : fi;
-          loss += (float)out_meta[i] * (fmaxf(z, 0.f) + log1pf(__expf(-fabsf(z))));
-        }
-      }
-    }
-  }
+// ---- the persistent engine's rows and step arithmetic ---------------------------------
+// The persistent kernels keep a step's rows in shared memory in quarters: when d % 16 == 0,
+// a row is four quarters of d / 4 columns, each followed by 4 words of padding, else d
+// columns and 4 words.  Shared memory returns 128 bytes per cycle to the registers of an SM
+// whatever the lanes' addresses, and that, not FMA issue, bounded these kernels, so the
+// layout serves the forward's register tiles: lanes that hold the four quarters of a row
+// and two neighbouring rows read 8 distinct 16-byte bank groups (the row stride is 4 groups
+// modulo 8).
+struct RowShape {
+  int stride;  // words from row to row
+  int q4;      // 4-column chunks per quarter (d % 16 == 0), else d / 4: one range
+};
+__host__ __device__ __forceinline__ RowShape row_shape(int d) {
+  return (d & 15) == 0 ? RowShape{d + 16, d >> 4} : RowShape{d + 4, d >> 2};
+}
+// word offset of chunk q's 4 columns in a row
+__device__ __forceinline__ int chunk_at(int q, const RowShape& R) { return 4 * (q + q / R.q4); }
+
+// The reference's gradient of one dot product (dsgl.hpp:1243-1272), without branches: past
+// +-6 the sigmoid is 1 or 0, and label - 1, label - 0 are exact.
+__device__ __forceinline__ float step_gradient(float f, int label, const float* exp_table, float alpha, int meta) {
+  const int idx = __float2int_rz(__fmul_rn(__fadd_rn(f, (float)kMaxExp), (float)kTableScale));
+  float sig = exp_table[min(max(idx, 0), kExpTableSize)];
+  sig = f > (float)kMaxExp ? 1.f : f < -(float)kMaxExp ? 0.f : sig;
+  return __fmul_rn(__fmul_rn(__fsub_rn((float)label, sig), alpha), (float)meta);
+}
+__device__ __forceinline__ float step_loss(float f, int label, int meta) {
+  const float z = label ? -f : f;
+  return (float)meta * (fmaxf(z, 0.f) + log1pf(__expf(-fabsf(z))));
 }
 
-// The split forward with two lanes per input while at most 16 inputs remain (each lane sums
-// two of the four quarters): half the k-loop per lane for those rounds, the same bits.
-template <int OM, class InPtr>
-__device__ __forceinline__ void forward_gradient_two_lanes(int I, int first, int O, int d, InPtr in_ptr,
-                                                        const float* out_rows, int DP, const int* out_meta,
-                                                        const float* exp_table, float alpha, float2* corrP,
-                                                        bool want_loss, float& loss) {
+// Forward of one warp's step: every dot product is eight sequential partial sums -- the even
+// and the odd k of each quarter of [0, d), each pair advanced by one FFMA2 on
+// {o[k], o[k+1]} x {x[k], x[k+1]} -- combined as s_m = even_m + odd_m,
+// f = (s_0 + s_1) + (s_2 + s_3) when d % 16 == 0; when not, [0, d) is one range and
+// f = even + odd.  The oracle's window policy uses the same order.
+// Register tiles: with quarters, lane = m + 4 og + 8 ig holds quarter m of TI inputs
+// (j0 + ig + 4 t) against the outputs of parity og, so a chunk of TI + TO rows read feeds
+// TI TO products (against 8 reads for 7 with one lane per input and the outputs broadcast);
+// the quarters' sums meet by shuffles, (s_0 + s_1) first, each lane keeping a part.  One
+// range: lane = og + 2 ig, two inputs each.
+// corr[j * CS + i] = g_ij, CS = OM rounded up to 4.
+template <int OM, int DFIX, class InPtr>
+__device__ __forceinline__ void forward_tiled(int I, int first, int O, int d_rt, InPtr in_ptr, const float* out_rows,
+                                              const int* out_meta, const float* exp_table, float alpha, float* corr,
+                                              bool want_loss, float& loss) {
+  constexpr int CS = (OM + 3) & ~3, TO = (OM + 1) / 2;
+  const int d = DFIX ? DFIX : d_rt;
+  const RowShape R = row_shape(d);
+  const int lane = lane_id();
+  auto finish = [&](int j, int i, float f) {
+    if (j < I && i < O) {
+      const int label = j < first ? (i == 0) : (i == 1);  // outputs t1, t2, negatives
+      corr[j * CS + i] = step_gradient(f, label, exp_table, alpha, out_meta[i]);
+      if (want_loss) loss += step_loss(f, label, out_meta[i]);
+    }
+  };
   if ((d & 15) == 0) {
-    const int q4 = d >> 4;
-    for (int j0 = 0; j0 < I;) {
-      const int rem = I - j0;
-      if (rem <= 16) {
-        forward_round<2, 2, false, OM>(j0, rem, first, O, q4, in_ptr, out_rows, DP, out_meta, exp_table, alpha,
-                                       corrP, want_loss, loss);
-        j0 += rem;
-      } else {
-        const int nj = rem < 32 ? rem : 32;
-        forward_round<4, 1, false, OM>(j0, nj, first, O, q4, in_ptr, out_rows, DP, out_meta, exp_table, alpha,
-                                       corrP, want_loss, loss);
-        j0 += nj;
+    constexpr int TI = 4;
+    const int m = lane & 3, og = (lane >> 2) & 1, ig = lane >> 3;
+    const int q4 = R.q4, at = 4 * m * (q4 + 1);  // the quarter's first word
+    // output rows og, og + 2, ..; one past OM is read as the first (an unused sum)
+    const float* o0 = out_rows + og * R.stride + at;
+    const int last = 2 * (TO - 1) + og < OM ? 2 * (TO - 1) * R.stride : 0;
+    for (int j0 = 0; j0 < I; j0 += 4 * TI) {
+      const float4* x[TI];
+#pragma unroll
+      for (int t = 0; t < TI; t++) {
+        const int j = j0 + ig + 4 * t;
+        x[t] = reinterpret_cast<const float4*>(in_ptr(j < I ? j : I - 1) + at);
+      }
+      float2 f[TI][TO];
+#pragma unroll
+      for (int t = 0; t < TI; t++)
+#pragma unroll
+        for (int u = 0; u < TO; u++) f[t][u] = make_float2(0.f, 0.f);
+#pragma unroll 2
+      for (int k4 = 0; k4 < q4; k4++) {
+        float4 xv[TI], ov[TO];  // rows past O hold stale data: unused sums
+#pragma unroll
+        for (int t = 0; t < TI; t++) xv[t] = x[t][k4];
+#pragma unroll
+        for (int u = 0; u < TO; u++)
+          ov[u] = reinterpret_cast<const float4*>(o0 + (u < TO - 1 ? 2 * u * R.stride : last))[k4];
+#pragma unroll
+        for (int t = 0; t < TI; t++)
+#pragma unroll
+          for (int u = 0; u < TO; u++)
+            f[t][u] = ffma2(make_float2(ov[u].x, ov[u].y), make_float2(xv[t].x, xv[t].y), f[t][u]);
+#pragma unroll
+        for (int t = 0; t < TI; t++)
+#pragma unroll
+          for (int u = 0; u < TO; u++)
+            f[t][u] = ffma2(make_float2(ov[u].z, ov[u].w), make_float2(xv[t].z, xv[t].w), f[t][u]);
+      }
+      // quarters (0, 1) and (2, 3) meet: lanes of even m keep inputs t = 0, 1, of odd m 2, 3;
+      // then the two halves: m < 2 keeps the first of its two inputs, m >= 2 the second
+      float s[2][TO];
+#pragma unroll
+      for (int t = 0; t < 2; t++)
+#pragma unroll
+        for (int u = 0; u < TO; u++) {
+          const float a = __fadd_rn(f[t][u].x, f[t][u].y), b = __fadd_rn(f[t + 2][u].x, f[t + 2][u].y);
+          const float got = __shfl_xor_sync(kFull, (m & 1) ? a : b, 1);
+          s[t][u] = __fadd_rn((m & 1) ? b : a, got);
+        }
+      const int j = j0 + ig + 4 * (2 * (m & 1) + (m >> 1));
+#pragma unroll
+      for (int u = 0; u < TO; u++) {
+        const float got = __shfl_xor_sync(kFull, (m & 2) ? s[0][u] : s[1][u], 2);
+        finish(j, 2 * u + og, __fadd_rn((m & 2) ? s[1][u] : s[0][u], got));
       }
     }
   } else {
-    for (int j0 = 0; j0 < I; j0 += 32)
-      forward_round<1, 1, true, OM>(j0, I - j0 < 32 ? I - j0 : 32, first, O, d >> 2, in_ptr, out_rows, DP,
-                                    out_meta, exp_table, alpha, corrP, want_loss, loss);
-  }
-  __syncwarp();
-}
-
-template <int OM, class InPtr>
-__device__ __forceinline__ void forward_gradient_split8(int I, int first, int O, int d, InPtr in_ptr,
-                                                        const float* out_rows, int DP, const int* out_meta,
-                                                        const float* exp_table, float alpha, float2* corrP,
-                                                        bool want_loss, float& loss) {
-  typedef StepShape<OM> SS;
-  const int lane = lane_id();
-  const int nq = (d & 15) == 0 ? 4 : 1;  // quarters of [0, d) (one range when d % 16 != 0)
-  const int q4 = (d >> 2) / nq;          // chunks of 4 columns per quarter
-  for (int j0 = 0; j0 < I; j0 += 32) {
-    const int j = j0 + lane;
-    const float4* x = reinterpret_cast<const float4*>(in_ptr(j < I ? j : I - 1));
-    float2 f[OM][4];
+    constexpr int TI = 2;
+    const int og = lane & 1, ig = lane >> 1;
+    const float* o0 = out_rows + og * R.stride;
+    const int last = 2 * (TO - 1) + og < OM ? 2 * (TO - 1) * R.stride : 0;
+    for (int j0 = 0; j0 < I; j0 += 16 * TI) {
+      const float4* x[TI];
 #pragma unroll
-    for (int i = 0; i < OM; i++)
-#pragma unroll
-      for (int m = 0; m < 4; m++) f[i][m] = make_float2(0.f, 0.f);
-    for (int k4 = 0; k4 < q4; k4++) {
-      float4 xv[4];
-#pragma unroll
-      for (int m = 0; m < 4; m++) xv[m] = m < nq ? x[m * q4 + k4] : make_float4(0.f, 0.f, 0.f, 0.f);
-      // Rows i >= O hold stale but readable data; their sums are never used, so the loop
-      // runs over all OM rows without a branch.
-#pragma unroll
-      for (int i = 0; i < OM; i++) {
-        const float4* orow = reinterpret_cast<const float4*>(out_rows + (size_t)i * DP);
-#pragma unroll
-        for (int m = 0; m < 4; m++) {
-          if (m >= nq) continue;
-          const float4 o = orow[m * q4 + k4];
-          f[i][m] = ffma2(make_float2(o.x, o.y), make_float2(xv[m].x, xv[m].y), f[i][m]);
-          f[i][m] = ffma2(make_float2(o.z, o.w), make_float2(xv[m].z, xv[m].w), f[i][m]);
-        }
+      for (int t = 0; t < TI; t++) {
+        const int j = j0 + ig + 16 * t;
+        x[t] = reinterpret_cast<const float4*>(in_ptr(j < I ? j : I - 1));
       }
-    }
-    if (j < I) {
+      float2 f[TI][TO];
 #pragma unroll
-      for (int i = 0; i < OM; i++) {
-        if (i < O) {
-          const int label = j < first ? (i == 0) : (i == 1);  // outputs t1, t2, negatives
-          const float s0 = __fadd_rn(f[i][0].x, f[i][0].y), s1 = __fadd_rn(f[i][1].x, f[i][1].y);
-          const float s2 = __fadd_rn(f[i][2].x, f[i][2].y), s3 = __fadd_rn(f[i][3].x, f[i][3].y);
-          const float fi = __fadd_rn(__fadd_rn(s0, s1), __fadd_rn(s2, s3));
-          float g;
-          if (fi > (float)kMaxExp) {
-            g = __fmul_rn((float)(label - 1), alpha);
-          } else if (fi < -(float)kMaxExp) {
-            g = __fmul_rn((float)label, alpha);
-          } else {
-            const int idx =
-                __float2int_rz(__fmul_rn(__fadd_rn(fi, (float)kMaxExp), (float)kTableScale));
-            g = __fmul_rn(__fsub_rn((float)label, exp_table[idx]), alpha);
+      for (int t = 0; t < TI; t++)
+#pragma unroll
+        for (int u = 0; u < TO; u++) f[t][u] = make_float2(0.f, 0.f);
+#pragma unroll 2
+      for (int k4 = 0; k4 < R.q4; k4++) {
+        float4 xv[TI], ov[TO];
+#pragma unroll
+        for (int t = 0; t < TI; t++) xv[t] = x[t][k4];
+#pragma unroll
+        for (int u = 0; u < TO; u++)
+          ov[u] = reinterpret_cast<const float4*>(o0 + (u < TO - 1 ? 2 * u * R.stride : last))[k4];
+#pragma unroll
+        for (int t = 0; t < TI; t++)
+#pragma unroll
+          for (int u = 0; u < TO; u++) {
+            f[t][u] = ffma2(make_float2(ov[u].x, ov[u].y), make_float2(xv[t].x, xv[t].y), f[t][u]);
+            f[t][u] = ffma2(make_float2(ov[u].z, ov[u].w), make_float2(xv[t].z, xv[t].w), f[t][u]);
           }
-          const float gm = __fmul_rn(g, (float)out_meta[i]);
-          corrP[j * SS::CS + i] = make_float2(gm, gm);
-          if (want_loss) {
-            const float z = label ? -fi : fi;
-            loss += (float)out_meta[i] * (fmaxf(z, 0.f) + log1pf(__expf(-fabsf(z))));
-          }
-        }
       }
+#pragma unroll
+      for (int t = 0; t < TI; t++)
+#pragma unroll
+        for (int u = 0; u < TO; u++)
+          // the sum's three empty partners of the eight-sum form
+          finish(j0 + ig + 16 * t, 2 * u + og, __fadd_rn(__fadd_rn(__fadd_rn(f[t][u].x, f[t][u].y), 0.f), 0.f));
     }
   }
   __syncwarp();
-}
-
-// Stores the step's output rows from registers in the normal layout (stride DP).
-template <int OM, int DCH>
-__device__ __forceinline__ void store_out_normal(const float4 (&v)[OM][DCH], int O, int d, float* out_rows,
-                                                 int DP) {
-  const int lane = lane_id(), d4 = d >> 2;
-#pragma unroll
-  for (int t = 0; t < DCH; t++) {
-    const int q = lane + 32 * t;
-    if (q < d4) {
-#pragma unroll
-      for (int i = 0; i < OM; i++)
-        if (i < O) reinterpret_cast<float4*>(out_rows + (size_t)i * DP)[q] = v[i][t];
-    }
-  }
 }
 
 // Backward.  Lane owns column chunks q = lane + 32 t (t < DCH, q < d/4), as two pairs.
@@ -573,9 +537,7 @@ __device__ __forceinline__ void store_out_normal(const float4 (&v)[OM][DCH], int
 // md is complete before any input row changes, as the reference's two GEMMs read the
 // same pre-update inputM.  apply_in(j, q, a) consumes input j's update of chunk q.
 // out_pair(p, q, r0, r1): rows 2p and 2p+1 of the step's outputs, columns 4q..4q+3.
-// kT2Second: outputs are stored t1, t2, negatives (select_outputs); the sum over i still
-// runs in the reference's order t1, negatives, t2, i.e. stored rows 0, 2..O-1, 1.
-template <int OM, int DCH, bool kT2Second = false, class InPtr, class OutPair, class ApplyIn>
+template <int OM, int DCH, class InPtr, class OutPair, class ApplyIn>
 __device__ __forceinline__ void backward(int I, int O, int d, InPtr in_ptr, OutPair out_pair,
                                          const float2* corrP, float4 (&md)[OM][DCH], ApplyIn apply_in) {
   typedef StepShape<OM> SS;
@@ -653,11 +615,8 @@ __device__ __forceinline__ void backward(int I, int O, int d, InPtr in_ptr, OutP
 #pragma unroll
         for (int u = 0; u < 4; u++) al[u] = ah[u] = make_float2(0.f, 0.f);
 #pragma unroll
-        for (int k = 0; k < OM; k++) {
-          // k-th term in the reference's order, as a stored row index (t2 comes last)
-          const int i = !kT2Second ? k : (k == 0 ? 0 : (k == OM - 1 ? 1 : k + 1));
-          const bool used = !kT2Second ? k < O : (k == 0 || k == OM - 1 || k + 1 < O);
-          if (used) {
+        for (int i = 0; i < OM; i++) {
+          if (i < O) {
 #pragma unroll
             for (int u = 0; u < 4; u++) {
               al[u] = ffma2(c[u][i], olo[i][t], al[u]);
@@ -674,79 +633,171 @@ __device__ __forceinline__ void backward(int I, int O, int d, InPtr in_ptr, OutP
   __syncwarp();
 }
 
-// The same backward in one pass over the inputs, for steps in which no two inputs share a
-// row: input j's row is read for outputMd and then updated, and no later input reads it,
-// so every accumulator sees the same operands in the same order as backward<> above (md
-// sequential in j, each input's update summed over the outputs in the reference's order,
-// then added to the row).  One pass loads each input row and its coefficients once.
-template <int OM, int DCH, bool kT2Second = false, class InPtr, class OutPair>
-__device__ __forceinline__ void backward_merged(int I, int O, int d, InPtr in_ptr, OutPair out_pair,
-                                                const float2* corrP, float4 (&md)[OM][DCH]) {
-  typedef StepShape<OM> SS;
-  const int lane = lane_id();
-  const int d4 = d >> 2;
-  float2 olo[SS::OMP][DCH], ohi[SS::OMP][DCH];
+// Backward of the persistent kernels.  A lane owns NC pairs of columns of every row: one pair
+// (2 columns), a chunk of 4, or two chunks `step` words apart.
+//   m_i  = sum_j g_ij x_j     (outputMd, dsgl.hpp:1290), sequential in j
+//   x_j += sum_i g_ij o_i     (dsgl.hpp:1309-1333), in the reference's order t1, negatives, t2
+//                             (stored rows 0, 2 .. O-1, 1)
+// outputMd is summed over rows no input has changed yet: in one pass when no two inputs share
+// a row (an input's row is read for outputMd, then updated), else before any update.
+template <int NC>
+__device__ __forceinline__ void load_cols(const float* p, int step, float2 (&v)[NC]) {
+  if constexpr (NC == 1) {
+    v[0] = *reinterpret_cast<const float2*>(p);
+  } else {
 #pragma unroll
-  for (int pp = 0; pp < SS::NPAIR; pp++)
-#pragma unroll
-    for (int t = 0; t < DCH; t++) {
-      const int q = lane + 32 * t;
-      float4 r0 = make_float4(0.f, 0.f, 0.f, 0.f), r1 = r0;
-      if (2 * pp < O && q < d4) out_pair(pp, q, r0, r1);
-      olo[2 * pp][t] = make_float2(r0.x, r0.y);
-      ohi[2 * pp][t] = make_float2(r0.z, r0.w);
-      olo[2 * pp + 1][t] = make_float2(r1.x, r1.y);
-      ohi[2 * pp + 1][t] = make_float2(r1.z, r1.w);
-    }
-  float2 mlo[OM][DCH], mhi[OM][DCH];
-#pragma unroll
-  for (int i = 0; i < OM; i++)
-#pragma unroll
-    for (int t = 0; t < DCH; t++) mlo[i][t] = mhi[i][t] = make_float2(0.f, 0.f);
-  float4* x_next = I > 0 ? reinterpret_cast<float4*>(const_cast<float*>(in_ptr(0))) : nullptr;
-  for (int j = 0; j < I; j++) {
-    float4* x = x_next;
-    x_next = reinterpret_cast<float4*>(const_cast<float*>(in_ptr(j + 1 < I ? j + 1 : j)));
-    const float4* cj = reinterpret_cast<const float4*>(corrP + j * SS::CS);
-    float2 c[SS::OMP];
-#pragma unroll
-    for (int q = 0; q < SS::NPAIR; q++) {
-      const float4 v = cj[q];
-      c[2 * q] = make_float2(v.x, v.y);
-      c[2 * q + 1] = make_float2(v.z, v.w);
-    }
-#pragma unroll
-    for (int t = 0; t < DCH; t++) {
-      const int q = lane + 32 * t;
-      if (q < d4) {
-        const float4 xv = x[q];
-        const float2 xl = make_float2(xv.x, xv.y), xh = make_float2(xv.z, xv.w);
-#pragma unroll
-        for (int i = 0; i < OM; i++)
-          if (i < O) {
-            mlo[i][t] = ffma2(c[i], xl, mlo[i][t]);
-            mhi[i][t] = ffma2(c[i], xh, mhi[i][t]);
-          }
-        float2 al = make_float2(0.f, 0.f), ah = al;
-#pragma unroll
-        for (int k = 0; k < OM; k++) {
-          const int i = !kT2Second ? k : (k == 0 ? 0 : (k == OM - 1 ? 1 : k + 1));
-          const bool used = !kT2Second ? k < O : (k == 0 || k == OM - 1 || k + 1 < O);
-          if (used) {
-            al = ffma2(c[i], olo[i][t], al);
-            ah = ffma2(c[i], ohi[i][t], ah);
-          }
-        }
-        const float2 lo = fadd2(xl, al), hi = fadd2(xh, ah);
-        x[q] = make_float4(lo.x, lo.y, hi.x, hi.y);
-      }
+    for (int k = 0; k < NC / 2; k++) {
+      const float4 t = *reinterpret_cast<const float4*>(p + k * step);
+      v[2 * k] = make_float2(t.x, t.y), v[2 * k + 1] = make_float2(t.z, t.w);
     }
   }
+}
+template <int NC>
+__device__ __forceinline__ void store_cols(float* p, int step, const float2 (&v)[NC]) {
+  if constexpr (NC == 1) {
+    *reinterpret_cast<float2*>(p) = v[0];
+  } else {
 #pragma unroll
-  for (int i = 0; i < OM; i++)
+    for (int k = 0; k < NC / 2; k++)
+      *reinterpret_cast<float4*>(p + k * step) = make_float4(v[2 * k].x, v[2 * k].y, v[2 * k + 1].x, v[2 * k + 1].y);
+  }
+}
+// gradients of input j for N outputs from i0 (a multiple of 2; of 4 when N > 2)
+template <int OM, int N>
+__device__ __forceinline__ void load_coef(const float* corr, int j, int i0, float (&c)[N]) {
+  constexpr int CS = (OM + 3) & ~3;
+  const float* cj = corr + j * CS + i0;
+  if constexpr (N % 4 == 2) {  // i0 may be 2 past a multiple of 4
 #pragma unroll
-    for (int t = 0; t < DCH; t++) md[i][t] = make_float4(mlo[i][t].x, mlo[i][t].y, mhi[i][t].x, mhi[i][t].y);
-  __syncwarp();
+    for (int k = 0; k < N / 2; k++) {
+      const float2 v = reinterpret_cast<const float2*>(cj)[k];
+      c[2 * k] = v.x, c[2 * k + 1] = v.y;
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < (N + 3) / 4; k++) {
+      const float4 v = reinterpret_cast<const float4*>(cj)[k];
+      const float e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int t = 0; t < 4; t++)
+        if (4 * k + t < N) c[4 * k + t] = e[t];
+    }
+  }
+}
+template <int N, int NC>
+__device__ __forceinline__ void accumulate_out(const float (&c)[N], const float2 (&x)[NC], float2 (&m)[N][NC]) {
+#pragma unroll
+  for (int i = 0; i < N; i++)
+#pragma unroll
+    for (int t = 0; t < NC; t++) m[i][t] = ffma2(make_float2(c[i], c[i]), x[t], m[i][t]);
+}
+// an input's addend, sum_i g_ij o_i in the reference's order.  kAll: O == OM
+template <int OM, int NC, bool kAll>
+__device__ __forceinline__ void input_addend(const float (&c)[OM], const float2 (&o)[OM][NC], int O, float2 (&a)[NC]) {
+#pragma unroll
+  for (int t = 0; t < NC; t++) a[t] = ffma2(make_float2(c[0], c[0]), o[0][t], make_float2(0.f, 0.f));
+#pragma unroll
+  for (int i = 2; i < OM; i++)
+    if (kAll || i < O) {
+#pragma unroll
+      for (int t = 0; t < NC; t++) a[t] = ffma2(make_float2(c[i], c[i]), o[i][t], a[t]);
+    }
+#pragma unroll
+  for (int t = 0; t < NC; t++) a[t] = ffma2(make_float2(c[1], c[1]), o[1][t], a[t]);
+}
+template <int OM, int NC, bool kAll>
+__device__ __forceinline__ void update_input(const float (&c)[OM], const float2 (&o)[OM][NC], int O, float2 (&x)[NC]) {
+  float2 a[NC];
+  input_addend<OM, NC, kAll>(c, o, O, a);
+#pragma unroll
+  for (int t = 0; t < NC; t++) x[t] = fadd2(x[t], a[t]);
+}
+// outputMd of N outputs from i0 over all inputs; x: the rows at the lane's columns
+template <int OM, int N, int NC>
+__device__ __forceinline__ void step_out_md(int I, const float* x, int step, const int* in_off, const float* corr, int i0,
+                                            float2 (&m)[N][NC]) {
+  int j = 0;
+  for (; j + 4 <= I; j += 4) {
+    const int4 off = *reinterpret_cast<const int4*>(in_off + j);
+    float2 xv[4][NC];
+    float c[4][N];
+    load_cols<NC>(x + off.x, step, xv[0]);
+    load_cols<NC>(x + off.y, step, xv[1]);
+    load_cols<NC>(x + off.z, step, xv[2]);
+    load_cols<NC>(x + off.w, step, xv[3]);
+#pragma unroll
+    for (int u = 0; u < 4; u++) load_coef<OM, N>(corr, j + u, i0, c[u]);
+#pragma unroll
+    for (int u = 0; u < 4; u++) accumulate_out<N, NC>(c[u], xv[u], m);
+  }
+  for (; j < I; j++) {
+    float2 xv[NC];
+    float c[N];
+    load_cols<NC>(x + in_off[j], step, xv);
+    load_coef<OM, N>(corr, j, i0, c);
+    accumulate_out<N, NC>(c, xv, m);
+  }
+}
+// updates of inputs [j0, j1), in order
+template <int OM, int NC, bool kAll>
+__device__ __forceinline__ void step_update(int j0, int j1, int O, bool distinct, float* x, int step, const int* in_off,
+                                            const float* corr, const float2 (&o)[OM][NC]) {
+  int j = j0;
+  if (__builtin_expect(distinct, 1)) {
+    for (; j + 2 <= j1; j += 2) {
+      float *xa = x + in_off[j], *xb = x + in_off[j + 1];
+      float2 va[NC], vb[NC];
+      float ca[OM], cb[OM];
+      load_cols<NC>(xa, step, va);
+      load_cols<NC>(xb, step, vb);
+      load_coef<OM, OM>(corr, j, 0, ca);
+      load_coef<OM, OM>(corr, j + 1, 0, cb);
+      update_input<OM, NC, kAll>(ca, o, O, va);
+      update_input<OM, NC, kAll>(cb, o, O, vb);
+      store_cols<NC>(xa, step, va);
+      store_cols<NC>(xb, step, vb);
+    }
+  }
+  for (; j < j1; j++) {
+    float* xa = x + in_off[j];
+    float2 va[NC];
+    float ca[OM];
+    load_cols<NC>(xa, step, va);
+    load_coef<OM, OM>(corr, j, 0, ca);
+    update_input<OM, NC, kAll>(ca, o, O, va);
+    store_cols<NC>(xa, step, va);
+  }
+}
+// both products over all inputs, for steps without shared rows
+template <int OM, int NC, bool kAll>
+__device__ __forceinline__ void step_merged(int I, int O, float* x, int step, const int* in_off, const float* corr,
+                                            const float2 (&o)[OM][NC], float2 (&m)[OM][NC]) {
+  int j = 0;
+  for (; j + 2 <= I; j += 2) {
+    const int2 off = *reinterpret_cast<const int2*>(in_off + j);
+    float2 va[NC], vb[NC];
+    float ca[OM], cb[OM];
+    load_cols<NC>(x + off.x, step, va);
+    load_cols<NC>(x + off.y, step, vb);
+    load_coef<OM, OM>(corr, j, 0, ca);
+    load_coef<OM, OM>(corr, j + 1, 0, cb);
+    accumulate_out<OM, NC>(ca, va, m);
+    update_input<OM, NC, kAll>(ca, o, O, va);
+    store_cols<NC>(x + off.x, step, va);
+    accumulate_out<OM, NC>(cb, vb, m);
+    update_input<OM, NC, kAll>(cb, o, O, vb);
+    store_cols<NC>(x + off.y, step, vb);
+  }
+  if (j < I) {
+    float* xa = x + in_off[j];
+    float2 va[NC];
+    float ca[OM];
+    load_cols<NC>(xa, step, va);
+    load_coef<OM, OM>(corr, j, 0, ca);
+    accumulate_out<OM, NC>(ca, va, m);
+    update_input<OM, NC, kAll>(ca, o, O, va);
+    store_cols<NC>(xa, step, va);
+  }
 }
 
 // Stores the step's output rows from registers in the interleaved layout (see StepShape).
@@ -788,22 +839,6 @@ struct AddToInput {
 template <class InPtr>
 __device__ __forceinline__ AddToInput<InPtr> add_to_input(InPtr f) {
   return AddToInput<InPtr>{f};
-}
-
-// Loads the step's output rows (all loads in flight before any use) into registers.
-template <int S, int OM, int DCH>
-__device__ __forceinline__ void load_out_rows(const void* tab, const int* ids, int O, int d,
-                                              float4 (&v)[OM][DCH]) {
-  const int lane = lane_id(), d4 = d >> 2;
-#pragma unroll
-  for (int i = 0; i < OM; i++) {
-    const int row = i < O ? ids[i] : 0;
-#pragma unroll
-    for (int t = 0; t < DCH; t++) {
-      const int q = lane + 32 * t;
-      v[i][t] = (i < O && q < d4) ? RowIO<S>::load4(tab, row, d, q) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-  }
 }
 
 }  // namespace sgns

@@ -11,11 +11,19 @@
 //     written back (stochastically rounded for bf16 tables) when it leaves it,
 //   * the step's output rows (target of each walk + shared negatives) and gradients;
 // the window bookkeeping (vertex and count of each slot, slot of each position) lives in
-// registers, one slot per lane.
+// registers, one slot per lane.  dsgl_team.cuh trains a worker with five warps instead; this
+// kernel is the faster one where workers fill the GPU (from about six per SM).
 // Negative rows are read from and added to Woh at each step, as the reference does for
 // the two target rows (dsgl.hpp:1346-1356).  Dot products of the forward are summed as
 // eight sequential partial sums (even and odd k of each quarter of [0, d)) combined
-// pairwise; the backward keeps the reference's order.  The negative pool keeps the reference's
+// pairwise, in register tiles (forward_tiled); the backward keeps the reference's order.
+// What bounds it: the dependent instruction stream of each worker at seven warps per SM
+// (shared memory 30 KB and about 240 registers per thread), then the 128 bytes per cycle that
+// shared memory returns to the registers.  The register tiles read a third of the bytes that
+// one lane per input did, and the gradients are kept once instead of as pairs: 1.1M vertices,
+// 1064 workers, d = 128: bf16 182.3 -> 159.7 ms a pass, d = 64 21.2 -> 16.7 (400k vertices).
+// A compact loop matters as much: batching or prefetching the backward's inputs four deep
+// cost 4-9% in instruction fetch.  The negative pool keeps the reference's
 // draw stream (max(len1,len2)*K draws per pool, group neg_count % n per step,
 // dsgl.hpp:1054-1073, 1136-1154) but is regenerated from its base LCG state instead of
 // being stored.
@@ -35,50 +43,45 @@ constexpr int kRing = 32;
 static_assert(kRing >= 2 * (kWMax - 1) + 2, "the ring must hold 2w + 2 positions for every allowed window");
 
 struct WinLayout {  // per-warp shared memory, in 4-byte words
-  int NS, DP, OP, OM, IM, lmax, outI;
+  int NS, DP, CS, OM, IM, lmax, outI;
   int rows, corr, sen, inrow, outid, outmeta, pend, words;
 };
 
 __host__ __device__ inline WinLayout win_layout(int d, int w, int K, int lmax) {
   WinLayout L;
-  L.NS = 2 * w + 2;  // resident slots per walk (2w+1 positions, +1 while a row enters)
-  L.DP = d + 4;      // padded row stride: 32 lanes reading 32 rows hit 32 distinct banks
+  L.NS = 2 * w + 1;  // resident rows per walk (an entering row may take the leaving one's slot)
+  L.DP = row_shape(d).stride;
   L.OM = K <= 5 ? 7 : kOMax;  // the kernel variant's output capacity (K + 2 <= OM)
-  L.OP = (L.OM + 1) & ~1;     // outputs rounded up to pairs
+  L.CS = (L.OM + 3) & ~3;     // a gradient row
   L.IM = 4 * w;
   L.lmax = lmax;
   int off = 0;
   L.rows = off;  // window rows of both walks
   off += 2 * L.NS * L.DP;
-  L.outI = off;  // the step's output rows, normal layout (stride DP)
-  off += L.OP * L.DP;
-  L.corr = off;  // duplicated gradient pairs, stride OP + 2 pairs per input
-  off += L.IM * (L.OP + 2) * 2;
+  L.outI = off;  // the step's output rows
+  off += L.OM * L.DP;
+  L.corr = off;
+  off += L.IM * L.CS;
+  L.inrow = off;  // row offsets (words) of the step's inputs
+  off += L.IM;
   L.sen = off;
   off += 2 * lmax;
-  L.inrow = off;
-  off += L.IM;
   L.outid = off;
   off += L.OM;
   L.outmeta = off;
   off += L.OM;
-  L.pend = off;  // pending row loads: ids, then destination rows
+  L.pend = off;  // pending row loads: ids, then destination offsets
   off += 2 * (w + 1);
   L.words = (off + 3) & ~3;
   return L;
 }
 
-template <int S>
-__device__ __forceinline__ void load_row_to_smem(const void* tab, int64_t row, int d, float* dst) {
-  const int d4 = d >> 2;
-  for (int q = lane_id(); q < d4; q += 32)
-    reinterpret_cast<float4*>(dst)[q] = RowIO<S>::load4(tab, row, d, q);
-}
 // Loads up to NB rows (ids[0..n)) into registers before storing any of them, so their
 // DRAM round trips overlap; dst(u) is the shared-memory row of the u-th id.
 template <int S, int DCH, int NB, class Dst>
 __device__ __forceinline__ void load_rows_batched(const void* tab, const int* ids, int n, int d, Dst dst) {
   const int lane = lane_id(), d4 = d >> 2;
+  const RowShape R = row_shape(d);
   for (int b0 = 0; b0 < n; b0 += NB) {
     float4 v[NB][DCH];
 #pragma unroll
@@ -95,11 +98,11 @@ __device__ __forceinline__ void load_rows_batched(const void* tab, const int* id
 #pragma unroll
     for (int u = 0; u < NB; u++) {
       if (b0 + u < n) {
-        float4* out = reinterpret_cast<float4*>(dst(b0 + u));
+        float* out = dst(b0 + u);
 #pragma unroll
         for (int t = 0; t < DCH; t++) {
           const int q = lane + 32 * t;
-          if (q < d4) out[q] = v[u][t];
+          if (q < d4) *reinterpret_cast<float4*>(out + chunk_at(q, R)) = v[u][t];
         }
       }
     }
@@ -110,18 +113,17 @@ template <int S>
 __device__ __forceinline__ void store_row_from_smem(void* tab, int64_t row, int d, const float* src,
                                                     uint64_t ev) {
   const int d4 = d >> 2;
+  const RowShape R = row_shape(d);
   for (int q = lane_id(); q < d4; q += 32)
-    RowIO<S>::store4(tab, row, d, q, reinterpret_cast<const float4*>(src)[q], ev);
+    RowIO<S>::store4(tab, row, d, q, *reinterpret_cast<const float4*>(src + chunk_at(q, R)), ev);
 }
 
 // kLoss: also accumulate the SGNS loss (compute_loss); without it no loss code is compiled
 // into the step.  DFIX: the hidden size as a compile-time constant (0: read from p.d).  With
 // d known, every shared-memory address of the step is a base register plus an immediate
 // offset and the column-range guards vanish; the arithmetic is the same either way.
-// TILE: lanes per input in the forward dot products (2: two lanes share an input while at
-// most 16 inputs remain; the same bits), chosen by the autotuner.  NW: windows per step (2,
-// the reference's step over two walks; 1, one walk per step).
-template <int S, int DCH, int OM, bool kLoss, int DFIX, int TILE, int NW = 2>
+// NW: windows per step (2, the reference's step over two walks; 1, one walk per step).
+template <int S, int DCH, int OM, bool kLoss, int DFIX, int NW = 2>
 __global__ void __launch_bounds__(256) window_engine_kernel(TrainParams p) {
   extern __shared__ __align__(16) float smem[];
   float* exp_s = smem;
@@ -147,14 +149,18 @@ __global__ void __launch_bounds__(256) window_engine_kernel(TrainParams p) {
   float* base = smem + kHdrWords + (threadIdx.x >> 5) * L.words;
   float* rows = base + L.rows;
   float* out_rows = base + L.outI;
-  float2* corrP = reinterpret_cast<float2*>(base + L.corr);
+  float* corr = base + L.corr;
   int* sen = reinterpret_cast<int*>(base + L.sen);
-  int* in_row = reinterpret_cast<int*>(base + L.inrow);
+  int* in_off = reinterpret_cast<int*>(base + L.inrow);
   int* out_id = reinterpret_cast<int*>(base + L.outid);
   int* out_meta = reinterpret_cast<int*>(base + L.outmeta);
   int* pend_id = reinterpret_cast<int*>(base + L.pend);
-  int* pend_row = pend_id + (w + 1);
+  int* pend_off = pend_id + (w + 1);
   const int NS = L.NS, DP = L.DP, lmax = L.lmax;
+  const RowShape R = row_shape(d);
+  // this lane's columns: chunk `lane` and, d > 128, the chunk `step` words after it
+  const int col = chunk_at(lane < (d >> 2) ? lane : 0, R);
+  const int step = DCH == 2 ? chunk_at(lane + 32 < (d >> 2) ? lane + 32 : lane, R) - col : 0;
 
   // dsgl.hpp:790-826
   uint64_t rng = (uint64_t)wid, word_count = 0, last_wc = 0, step_id = 0;
@@ -179,13 +185,12 @@ __global__ void __launch_bounds__(256) window_engine_kernel(TrainParams p) {
   // rows entering the windows at the last transition: loaded then, widened and stored to
   // their slots just before the next forward (so no instruction waits on the load earlier)
   typename RowIO<S>::Raw ent[2][DCH];
-  int ent_row[2] = {-1, -1};
+  int ent_off[2] = {-1, -1};
   // the next step's output rows, gathered at the end of this step when both walks go on
   // and the pool stays (ov_ready): the loads then overlap the window transitions.  Only
   // the variant with registers to spare for them across the transitions does this (bf16,
   // d <= 128, K <= 5: +3.7%; the fp32 rows are twice the registers and spill, -10%).
   constexpr bool kPrefetchRows = S == STORE_BF16 && DCH == 1 && OM == 7;
-  constexpr bool kMergedBackward = true;
   typename RowIO<S>::Raw ov[OM][DCH];
   bool ov_ready = false;
   int O_next = 0;
@@ -210,7 +215,7 @@ __global__ void __launch_bounds__(256) window_engine_kernel(TrainParams p) {
       const unsigned fr = __ballot_sync(kFull, lane < NS && my_r == 0);
       s = __ffs(fr) - 1;
       fresh = true;
-      if (s < 0) {  // cannot happen: at most 2w+2 distinct vertices are resident
+      if (s < 0) {  // cannot happen: a first window holds at most w + 1 rows
         if (lane == 0) atomicExch(&p.ctr->status, 2);
         s = 0;
       }
@@ -235,27 +240,15 @@ __global__ void __launch_bounds__(256) window_engine_kernel(TrainParams p) {
       if (fresh) {
         if (lane == 0) {
           pend_id[n] = v;
-          pend_row[n] = walk * NS + s;
+          pend_off[n] = (walk * NS + s) * DP;
         }
         n++;
       }
     }
     __syncwarp();
-    load_rows_batched<S, DCH, (DCH == 1 ? 8 : 4)>(p.wih, pend_id, n, d, [&](int u) { return rows + (size_t)pend_row[u] * DP; });
+    load_rows_batched<S, DCH, (DCH == 1 ? 8 : 4)>(p.wih, pend_id, n, d, [&](int u) { return rows + pend_off[u]; });
     n_loads += (unsigned long long)n;
     __syncwarp();
-  };
-  auto leave = [&](int walk, int position, uint64_t ev) {
-    const int s = __shfl_sync(kFull, walk ? rg1 : rg0, position & (kRing - 1));
-    const int r = __shfl_sync(kFull, walk ? sr1 : sr0, s) - 1;
-    const int v = __shfl_sync(kFull, walk ? sv1 : sv0, s);
-    if (lane == s) {
-      if (walk) sr1 = r; else sr0 = r;
-    }
-    if (r == 0) {
-      store_row_from_smem<S>(p.wih, v, d, rows + (size_t)(walk * NS + s) * DP, ev);
-      n_stores++;
-    }
   };
   auto flush_walk = [&](int walk, uint64_t ev) {
     const int my_r = walk ? sr1 : sr0, my_v = walk ? sv1 : sv0;
@@ -299,7 +292,7 @@ __global__ void __launch_bounds__(256) window_engine_kernel(TrainParams p) {
       last_wc = 0;
       cur = start;
       len[0] = len[1] = 0;
-      ent_row[0] = ent_row[1] = -1;
+      ent_off[0] = ent_off[1] = -1;
       sr0 = sr1 = 0;
       ov_ready = false;
       continue;
@@ -373,84 +366,93 @@ __global__ void __launch_bounds__(256) window_engine_kernel(TrainParams p) {
     }
     rng = lcg_next(rng);
     const int b = (int)fast_mod(rng, p.div_window);
-    const int I0 = window_inputs<true>(pos[0], len[0], w, b, 0, in_row,
-                                 [&](int c) { return __shfl_sync(kFull, rg0, c & (kRing - 1)); });
-    const int I = I0 + (two ? window_inputs<true>(pos[1], len[1], w, b, I0, in_row,
-                                                [&](int c) { return NS + __shfl_sync(kFull, rg1, c & (kRing - 1)); })
+    const int I0 = window_inputs<true>(pos[0], len[0], w, b, 0, in_off,
+                                 [&](int c) { return __shfl_sync(kFull, rg0, c & (kRing - 1)) * DP; });
+    const int I = I0 + (two ? window_inputs<true>(pos[1], len[1], w, b, I0, in_off,
+                                                [&](int c) { return (NS + __shfl_sync(kFull, rg1, c & (kRing - 1))) * DP; })
                             : 0);
 #pragma unroll
     for (int i = 0; i < OM; i++)
 #pragma unroll
-      for (int t = 0; t < DCH; t++) {
-        const int q = lane + 32 * t;
-        if (i < O && q < d4) reinterpret_cast<float4*>(out_rows + (size_t)i * DP)[q] = RowIO<S>::widen(ov[i][t]);
-      }
+      for (int t = 0; t < DCH; t++)
+        if (i < O && lane + 32 * t < d4)
+          *reinterpret_cast<float4*>(out_rows + i * DP + col + t * step) = RowIO<S>::widen(ov[i][t]);
 #pragma unroll
     for (int walk = 0; walk < 2; walk++) {
-      if (ent_row[walk] >= 0) {
-        float4* dst = reinterpret_cast<float4*>(rows + (size_t)ent_row[walk] * DP);
+      if (ent_off[walk] >= 0) {
 #pragma unroll
-        for (int t = 0; t < DCH; t++) {
-          const int q = lane + 32 * t;
-          if (q < (d >> 2)) dst[q] = RowIO<S>::widen(ent[walk][t]);
-        }
-        ent_row[walk] = -1;
+        for (int t = 0; t < DCH; t++)
+          if (lane + 32 * t < d4)
+            *reinterpret_cast<float4*>(rows + ent_off[walk] + col + t * step) = RowIO<S>::widen(ent[walk][t]);
+        ent_off[walk] = -1;
       }
     }
     __syncwarp();
     const float alpha = *reinterpret_cast<volatile float*>(&p.ctr->alpha);
-    auto in_ptr = [&](int j) -> const float* { return rows + (size_t)in_row[j] * DP; };
-    // two lanes per input for small rounds (d <= 128, K <= 5 only: the other variants have
-    // no registers to spare)
-    if (TILE == 2 && DCH == 1 && OM == 7)
-      forward_gradient_two_lanes<OM>(I, I0, O, d, in_ptr, out_rows, DP, out_meta, exp_s, alpha, corrP, kLoss, loss);
-    else
-      forward_gradient_split8<OM>(I, I0, O, d, in_ptr, out_rows, DP, out_meta, exp_s, alpha, corrP,
-                                  kLoss, loss);
-    float4 md[OM][DCH];
-    auto out_pair = [&](int pp, int q, float4& r0, float4& r1) {
-      r0 = reinterpret_cast<const float4*>(out_rows + (size_t)(2 * pp) * DP)[q];
-      r1 = 2 * pp + 1 < O ? reinterpret_cast<const float4*>(out_rows + (size_t)(2 * pp + 1) * DP)[q]
-                          : make_float4(0.f, 0.f, 0.f, 0.f);
-    };
+    forward_tiled<OM, DFIX>(I, I0, O, d, [&](int j) -> const float* { return rows + in_off[j]; }, out_rows, out_meta,
+                            exp_s, alpha, corr, kLoss, loss);
     // one pass over the inputs when no two of them share a window row (at most 32
-    // inputs, distinct slots); otherwise outputMd first, then the updates
-    bool merged = false;
-    if (kMergedBackward && I <= 32) {
-      const int r = lane < I ? in_row[lane] : -1 - lane;
-      merged = !__any_sync(kFull, __popc(__match_any_sync(kFull, r)) > 1);
+    // inputs, distinct rows); otherwise outputMd first, then the updates
+    bool distinct = false;
+    if (I <= 32) {
+      const int r = lane < I ? in_off[lane] : -1 - lane;
+      distinct = !__any_sync(kFull, __popc(__match_any_sync(kFull, r)) > 1);
     }
-    if (merged) backward_merged<OM, DCH, true>(I, O, d, in_ptr, out_pair, corrP, md);
-    else backward<OM, DCH, true>(I, O, d, in_ptr, out_pair, corrP, md, add_to_input(in_ptr));
-    {  // Woh += outputMd: target 1, target 2, then each negative (aliases follow that order)
-      uint64_t e1 = 0, e2 = 0, en = 0;
-      if (S == STORE_BF16) {
-        e1 = __shfl_sync(kFull, sr_key, EV_TARGET1);
-        e2 = __shfl_sync(kFull, sr_key, EV_TARGET2);
-        en = __shfl_sync(kFull, sr_key, EV_NEG);
-      }
-      const int d4 = d >> 2;
+    uint64_t e1 = 0, e2 = 0, en = 0;
+    if (S == STORE_BF16) {
+      e1 = __shfl_sync(kFull, sr_key, EV_TARGET1);
+      e2 = __shfl_sync(kFull, sr_key, EV_TARGET2);
+      en = __shfl_sync(kFull, sr_key, EV_NEG);
+    }
+    if (lane < d4) {
+      constexpr int NC = 2 * DCH;
+      // one pass holds the output rows and outputMd in registers: where they do not fit, the
+      // output rows are stored between the two products
+      constexpr bool kOnePass = OM * DCH <= 14;
+      const bool wide = DCH == 1 || lane + 32 < d4;  // the second chunk exists
+      float2 m[OM][NC];
 #pragma unroll
-      for (int t = 0; t < DCH; t++) {
-        const int q = lane + 32 * t;
-        if (q < d4) {
-          // outputs are stored t1, t2, negatives (see select_outputs)
-          const float4 b1 = reinterpret_cast<const float4*>(out_rows)[q];
-          const float4 n1 = RowIO<S>::store4(p.woh, t1, d, q, add4(b1, md[0][t]), e1);
-          float4 n2 = n1;
-          if (two) {
-            const float4 b2 = t2 == t1 ? n1 : reinterpret_cast<const float4*>(out_rows + DP)[q];
-            n2 = RowIO<S>::store4(p.woh, t2, d, q, add4(b2, md[1][t]), e2);
-          }
+      for (int i = 0; i < OM; i++)
 #pragma unroll
-          for (int i = 2; i < OM; i++) {
-            if (i < O) {
-              const int row = out_id[i];
-              const float4 bi = row == t2 ? n2 : reinterpret_cast<const float4*>(out_rows + (size_t)i * DP)[q];
-              RowIO<S>::store4(p.woh, row, d, q, add4(bi, md[i][t]), en);
+        for (int t = 0; t < NC; t++) m[i][t] = make_float2(0.f, 0.f);
+      // Woh += outputMd: target 1, target 2, then each negative (aliases follow that order;
+      // stored t1, t2, negatives, see select_outputs)
+      auto store_outputs = [&]() {
+#pragma unroll
+        for (int t = 0; t < DCH; t++) {
+          if (t == 0 || wide) {
+            const int q = lane + 32 * t;
+            auto base4 = [&](int i) { return *reinterpret_cast<const float4*>(out_rows + i * DP + col + t * step); };
+            auto md4 = [&](int i) { return make_float4(m[i][2 * t].x, m[i][2 * t].y, m[i][2 * t + 1].x, m[i][2 * t + 1].y); };
+            const float4 n1 = RowIO<S>::store4(p.woh, t1, d, q, add4(base4(0), md4(0)), e1);
+            float4 n2 = n1;
+            if (two) n2 = RowIO<S>::store4(p.woh, t2, d, q, add4(t2 == t1 ? n1 : base4(1), md4(1)), e2);
+#pragma unroll
+            for (int i = 2; i < OM; i++) {
+              if (i < O) {
+                const int row = out_id[i];
+                RowIO<S>::store4(p.woh, row, d, q, add4(row == t2 ? n2 : base4(i), md4(i)), en);
+              }
             }
           }
         }
+      };
+      float2 o[OM][NC];
+      auto load_outputs = [&]() {
+#pragma unroll
+        for (int i = 0; i < OM; i++) load_cols<NC>(out_rows + i * DP + col, step, o[i]);  // rows past O: unused
+      };
+      // (a lane without a second chunk runs its first one twice over: the same values)
+      if (kOnePass && __builtin_expect(distinct, 1)) {
+        load_outputs();
+        if (O == OM) step_merged<OM, NC, true>(I, O, rows + col, step, in_off, corr, o, m);
+        else step_merged<OM, NC, false>(I, O, rows + col, step, in_off, corr, o, m);
+        store_outputs();
+      } else {
+        step_out_md<OM, OM, NC>(I, rows + col, step, in_off, corr, 0, m);
+        store_outputs();
+        load_outputs();
+        step_update<OM, NC, false>(0, I, O, distinct, rows + col, step, in_off, corr, o);
       }
     }
     n_pairs += (unsigned long long)I;
@@ -485,7 +487,7 @@ __global__ void __launch_bounds__(256) window_engine_kernel(TrainParams p) {
       // to the slot just before the next forward, so the load overlaps the next step's
       // set-up.  A later write-back of the same vertex in this transition (walk 0's leave
       // or flush before walk 1's enter reads) is ordered after the load by program order.
-      const int d4 = d >> 2;
+#pragma unroll
       for (int walk = 0; walk < n_walks; walk++) {
         const uint64_t ev = S == STORE_BF16 ? __shfl_sync(kFull, sr_key, EV_WALK0 + walk) : 0;
         if (__builtin_expect(pos[walk] >= len[walk], 0)) {
@@ -493,22 +495,59 @@ __global__ void __launch_bounds__(256) window_engine_kernel(TrainParams p) {
           len[walk] = 0;
           train_sen_num++;
         } else {
+          int& my_v = walk ? sv1 : sv0;
+          int& my_r = walk ? sr1 : sr0;
+          int& my_g = walk ? rg1 : rg0;
           const int P = pos[walk];
+          // the leaving position's slot; its row leaves when no other position holds it and
+          // the entering position does not name the same vertex
+          int out_slot = -1, leave_v = -1, leave_off = 0;
+          bool out_last = false;
+          if (P - w - 1 >= 0) {
+            out_slot = __shfl_sync(kFull, my_g, (P - w - 1) & (kRing - 1));
+            out_last = __shfl_sync(kFull, my_r, out_slot) == 1;
+          }
           if (P + w < len[walk]) {
-            bool fresh;
-            int v;
-            const int s = enter_assign(walk, P + w, &fresh, &v);
+            const int v = sen[walk * lmax + P + w];
+            const unsigned hit = __ballot_sync(kFull, lane < NS && my_r > 0 && my_v == v);
+            const unsigned fr = __ballot_sync(kFull, lane < NS && (my_r == 0 || (out_last && lane == out_slot)));
+            const bool fresh = hit == 0;
+            int s = __ffs(fresh ? fr : hit) - 1;
+            if (s < 0) {  // cannot happen: 2w+1 positions stay
+              if (lane == 0) atomicExch(&p.ctr->status, 2);
+              s = 0;
+            }
             if (fresh) {
 #pragma unroll
-              for (int t = 0; t < DCH; t++) {
-                const int q = lane + 32 * t;
-                if (q < d4) ent[walk][t] = RowIO<S>::load_raw(p.wih, v, d, q);
-              }
-              ent_row[walk] = walk * NS + s;
+              for (int t = 0; t < DCH; t++)
+                if (lane + 32 * t < d4) ent[walk][t] = RowIO<S>::load_raw(p.wih, v, d, lane + 32 * t);
+              ent_off[walk] = (walk * NS + s) * DP;
               n_loads++;
             }
+            if (out_last && fresh && s == out_slot) {  // in the place of the row that leaves
+              leave_v = __shfl_sync(kFull, my_v, s);
+              leave_off = ent_off[walk];
+              if (lane == s) my_v = v;
+              out_slot = -1;
+            } else if (lane == s) {
+              my_v = v;
+              my_r++;
+            }
+            if (lane == ((P + w) & (kRing - 1))) my_g = s;
           }
-          if (P - w - 1 >= 0) leave(walk, P - w - 1, ev);
+          if (out_slot >= 0) {
+            const int r = __shfl_sync(kFull, my_r, out_slot) - 1;
+            const int v = __shfl_sync(kFull, my_v, out_slot);
+            if (lane == out_slot) my_r = r;
+            if (r == 0) {
+              leave_v = v;
+              leave_off = (walk * NS + out_slot) * DP;
+            }
+          }
+          if (leave_v >= 0) {
+            store_row_from_smem<S>(p.wih, leave_v, d, rows + leave_off, ev);
+            n_stores++;
+          }
         }
       }
     }
@@ -549,64 +588,51 @@ inline int fixed_d(int d) {
   return 0;
 }
 
-template <int S, int DCH, int OM, bool kLoss, int DFIX, int TILE>
+template <int S, int DCH, int OM, bool kLoss, int DFIX>
 static cudaError_t occupancy_d(int d, int w, int K, int lmax, int wpc, int* ctas) {
   const size_t smem = window_smem_bytes(d, w, K, lmax, wpc);
-  cudaError_t e = cudaFuncSetAttribute(window_engine_kernel<S, DCH, OM, kLoss, DFIX, TILE>,
+  cudaError_t e = cudaFuncSetAttribute(window_engine_kernel<S, DCH, OM, kLoss, DFIX>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas, window_engine_kernel<S, DCH, OM, kLoss, DFIX, TILE>,
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas, window_engine_kernel<S, DCH, OM, kLoss, DFIX>,
                                                        32 * wpc, smem);
 }
-template <int S, int DCH, int OM, int DFIX>
-static cudaError_t occupancy_tile(int d, int w, int K, int lmax, int wpc, int tile, int* ctas) {
-  if constexpr (DCH == 1 && OM == 7)
-    if (tile == 2) return occupancy_d<S, DCH, OM, false, DFIX, 2>(d, w, K, lmax, wpc, ctas);
-  return occupancy_d<S, DCH, OM, false, DFIX, 1>(d, w, K, lmax, wpc, ctas);
-}
 template <int S, int DCH, int OM>
-static cudaError_t occupancy_t(int d, int w, int K, int lmax, int wpc, int tile, int* ctas) {
+static cudaError_t occupancy_t(int d, int w, int K, int lmax, int wpc, int* ctas) {
   const int f = fixed_d(d);
   if constexpr (DCH == 1) {
-    if (f == 64) return occupancy_tile<S, DCH, OM, 64>(d, w, K, lmax, wpc, tile, ctas);
-    if (f == 128) return occupancy_tile<S, DCH, OM, 128>(d, w, K, lmax, wpc, tile, ctas);
+    if (f == 64) return occupancy_d<S, DCH, OM, false, 64>(d, w, K, lmax, wpc, ctas);
+    if (f == 128) return occupancy_d<S, DCH, OM, false, 128>(d, w, K, lmax, wpc, ctas);
   } else {
-    if (f == 256) return occupancy_tile<S, DCH, OM, 256>(d, w, K, lmax, wpc, tile, ctas);
+    if (f == 256) return occupancy_d<S, DCH, OM, false, 256>(d, w, K, lmax, wpc, ctas);
   }
-  return occupancy_tile<S, DCH, OM, 0>(d, w, K, lmax, wpc, tile, ctas);
+  return occupancy_d<S, DCH, OM, false, 0>(d, w, K, lmax, wpc, ctas);
 }
 
-template <int S, int DCH, int OM, bool kLoss, int DFIX, int TILE, int NW = 2>
+template <int S, int DCH, int OM, bool kLoss, int DFIX, int NW = 2>
 static cudaError_t launch_loss_t(const TrainParams& p, int wpc, cudaStream_t s) {
   const size_t smem = window_smem_bytes(p.d, p.window, p.K, p.lmax, wpc);
-  cudaError_t e = cudaFuncSetAttribute(window_engine_kernel<S, DCH, OM, kLoss, DFIX, TILE, NW>,
+  cudaError_t e = cudaFuncSetAttribute(window_engine_kernel<S, DCH, OM, kLoss, DFIX, NW>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   const int blocks = (p.workers + wpc - 1) / wpc;
-  window_engine_kernel<S, DCH, OM, kLoss, DFIX, TILE, NW><<<blocks, 32 * wpc, smem, s>>>(p);
+  window_engine_kernel<S, DCH, OM, kLoss, DFIX, NW><<<blocks, 32 * wpc, smem, s>>>(p);
   return cudaGetLastError();
-}
-template <int S, int DCH, int OM, bool kLoss, int DFIX>
-static cudaError_t launch_tile_t(const TrainParams& p, int wpc, cudaStream_t s) {
-  if constexpr (DCH == 1 && OM == 7)
-    if (p.fwd_tile == 2) return launch_loss_t<S, DCH, OM, kLoss, DFIX, 2>(p, wpc, s);
-  return launch_loss_t<S, DCH, OM, kLoss, DFIX, 1>(p, wpc, s);
 }
 template <int S, int DCH, int OM>
 static cudaError_t launch_t(const TrainParams& p, int wpc, cudaStream_t s) {
-  // single-window steps: the generic kernel (run-time d, one lane per input)
+  // single-window steps and the loss: the generic kernel (run-time d)
   if (p.windows == 1)
-    return p.compute_loss ? launch_loss_t<S, DCH, OM, true, 0, 1, 1>(p, wpc, s)
-                          : launch_loss_t<S, DCH, OM, false, 0, 1, 1>(p, wpc, s);
-  if (p.compute_loss) return launch_tile_t<S, DCH, OM, true, 0>(p, wpc, s);
+    return p.compute_loss ? launch_loss_t<S, DCH, OM, true, 0, 1>(p, wpc, s) : launch_loss_t<S, DCH, OM, false, 0, 1>(p, wpc, s);
+  if (p.compute_loss) return launch_loss_t<S, DCH, OM, true, 0>(p, wpc, s);
   const int f = fixed_d(p.d);
   if constexpr (DCH == 1) {
-    if (f == 64) return launch_tile_t<S, DCH, OM, false, 64>(p, wpc, s);
-    if (f == 128) return launch_tile_t<S, DCH, OM, false, 128>(p, wpc, s);
+    if (f == 64) return launch_loss_t<S, DCH, OM, false, 64>(p, wpc, s);
+    if (f == 128) return launch_loss_t<S, DCH, OM, false, 128>(p, wpc, s);
   } else {
-    if (f == 256) return launch_tile_t<S, DCH, OM, false, 256>(p, wpc, s);
+    if (f == 256) return launch_loss_t<S, DCH, OM, false, 256>(p, wpc, s);
   }
-  return launch_tile_t<S, DCH, OM, false, 0>(p, wpc, s);
+  return launch_loss_t<S, DCH, OM, false, 0>(p, wpc, s);
 }
 
 // kernel variants: storage x column chunks per lane (d <= 128 or <= 256) x outputs per
@@ -622,8 +648,8 @@ static cudaError_t launch_t(const TrainParams& p, int wpc, cudaStream_t s) {
     return small_ ? FN<STORE_F32, 1, 7>(__VA_ARGS__) : FN<STORE_F32, 1, kOMax>(__VA_ARGS__);                \
   } while (0)
 
-cudaError_t window_engine_occupancy(int storage, int d, int w, int K, int lmax, int wpc, int tile, int* ctas) {
-  SGNS_WINDOW_DISPATCH(occupancy_t, d, w, K, lmax, wpc, tile, ctas);
+cudaError_t window_engine_occupancy(int storage, int d, int w, int K, int lmax, int wpc, int* ctas) {
+  SGNS_WINDOW_DISPATCH(occupancy_t, d, w, K, lmax, wpc, ctas);
 }
 
 cudaError_t launch_window_engine(const TrainParams& p, int wpc, cudaStream_t s) {

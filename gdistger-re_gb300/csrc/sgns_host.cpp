@@ -65,6 +65,7 @@ struct sgns_handle {
   size_t plain_bytes = 0;
   // persistent engine launch shape and its captured graph
   int workers = 0, wpc = 0, tile = 1;
+  bool team = false;  // a team of warps trains each worker (else one warp)
   bool tuned = false;
   cudaGraphExec_t graph = nullptr;
   std::string graph_key;
@@ -336,7 +337,6 @@ TrainParams make_params(sgns_handle* h, int workers) {
   p.compute_loss = o.compute_loss;
   p.lmax = h->lmax;
   p.storage = o.storage == SGNS_STORE_BF16_SR ? STORE_BF16 : STORE_F32;
-  p.fwd_tile = h->tile;
   p.windows = o.windows_per_step == 1 ? 1 : 2;
   p.ctr = h->d_ctr;
   return p;
@@ -368,8 +368,8 @@ sgns_status finish_stats(sgns_handle* h, int workers, float ms) {
   s.workers = workers;
   s.warps_per_cta = h->opt.engine == SGNS_ENGINE_PERSISTENT ? h->wpc : 4;
   // single-window steps run the one-lane kernel
-  s.forward_tile = h->opt.engine != SGNS_ENGINE_PERSISTENT ? 0 : h->opt.windows_per_step == 1 ? 1 : h->tile;
-  s.warps_per_worker = 1;
+  s.forward_tile = h->opt.engine != SGNS_ENGINE_PERSISTENT ? 0 : h->opt.windows_per_step == 1 || h->team ? 1 : h->tile;
+  s.warps_per_worker = h->opt.engine == SGNS_ENGINE_PERSISTENT && h->team ? kTeamWarps : 1;
   s.row_loads = c.row_loads;
   s.row_stores = c.row_stores;
   s.output_rows = c.outputs;
@@ -380,8 +380,11 @@ sgns_status finish_stats(sgns_handle* h, int workers, float ms) {
 sgns_status persistent_shape(sgns_handle* h, int wpc, int* workers) {
   int ctas = 0;
   const sgns_options& o = h->opt;
-  CU(h, window_engine_occupancy(o.storage == SGNS_STORE_BF16_SR ? STORE_BF16 : STORE_F32, o.size,
-                                o.window, o.negative, h->lmax, wpc, h->tile, &ctas));
+  const int storage = o.storage == SGNS_STORE_BF16_SR ? STORE_BF16 : STORE_F32;
+  if (h->team)
+    CU(h, team_engine_occupancy(storage, o.size, o.window, o.negative, h->lmax, wpc, &ctas));
+  else
+    CU(h, window_engine_occupancy(storage, o.size, o.window, o.negative, h->lmax, wpc, &ctas));
   if (ctas < 1)
     return fail(h, SGNS_EINVAL, "a %d-warp CTA does not fit in shared memory (d=%d, walks up to %d)", wpc,
                 o.size, h->lmax);
@@ -396,12 +399,16 @@ sgns_status persistent_shape(sgns_handle* h, int wpc, int* workers) {
   return SGNS_OK;
 }
 
+cudaError_t launch_persistent(sgns_handle* h, const TrainParams& p, int wpc) {
+  return h->team ? launch_team_engine(p, wpc, h->stream) : launch_window_engine(p, wpc, h->stream);
+}
+
 sgns_status run_persistent(sgns_handle* h, int workers, int wpc, bool use_graph, float* ms_out) {
   TrainParams p = make_params(h, workers);
   if (use_graph) {
     char key[256];
-    snprintf(key, sizeof key, "%p/%lld/%d/%d/%p/%p/%d/%d/%d", (void*)h->d_corpus, (long long)h->n_tokens,
-             workers, wpc, h->wih, h->woh, h->lmax, h->opt.iter, h->tile);
+    snprintf(key, sizeof key, "%p/%lld/%d/%d/%p/%p/%d/%d/%d/%d", (void*)h->d_corpus, (long long)h->n_tokens,
+             workers, wpc, h->wih, h->woh, h->lmax, h->opt.iter, h->tile, (int)h->team);
     if (!h->graph || h->graph_key != key) {
       if (h->graph) cudaGraphExecDestroy(h->graph);
       h->graph = nullptr;
@@ -412,7 +419,7 @@ sgns_status run_persistent(sgns_handle* h, int workers, int wpc, bool use_graph,
       cudaGraph_t g;
       CU(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
       cudaError_t e1 = cudaMemcpyAsync(h->d_ctr, h->h_ctr, sizeof c, cudaMemcpyHostToDevice, h->stream);
-      cudaError_t e2 = launch_window_engine(p, wpc, h->stream);
+      cudaError_t e2 = launch_persistent(h, p, wpc);
       cudaError_t e3 = cudaStreamEndCapture(h->stream, &g);
       if (e1 != cudaSuccess || e2 != cudaSuccess || e3 != cudaSuccess)
         return fail(h, SGNS_ECUDA, "graph capture of the persistent launch failed: %s",
@@ -434,7 +441,7 @@ sgns_status run_persistent(sgns_handle* h, int workers, int wpc, bool use_graph,
     sgns_status st = reset_counters(h, workers);
     if (st) return st;
     CU(h, cudaEventRecord(h->ev0, h->stream));
-    CU(h, launch_window_engine(p, wpc, h->stream));
+    CU(h, launch_persistent(h, p, wpc));
     CU(h, cudaEventRecord(h->ev1, h->stream));
   }
   CU(h, cudaEventSynchronize(h->ev1));
@@ -490,8 +497,15 @@ std::string tune_key(const sgns_handle* h) {
     if (*c == '\t' || *c == '\n') *c = ' ';
   return key;
 }
-// "key<TAB>warps_per_cta<TAB>forward_tile" lines; the last entry for a key wins
-bool tune_cache_lookup(const std::string& key, int* wpc, int* tile) {
+// One launch shape of the persistent engine: a team of warps or one warp per worker, workers
+// per CTA, and the forward tile reported with the one-warp kernel.
+struct Shape {
+  bool team;
+  int wpc, tile;
+};
+// "key<TAB>warps_per_cta<TAB>forward_tile" lines, with a field "team" before them when teams
+// train the workers; the last entry for a key wins
+bool tune_cache_lookup(const std::string& key, Shape* out) {
   const char* path = getenv("SGNS_TUNE_CACHE");
   if (!path || !*path) return false;
   FILE* f = fopen(path, "r");
@@ -503,65 +517,78 @@ bool tune_cache_lookup(const std::string& key, int* wpc, int* tile) {
     if (!tab) continue;
     *tab = 0;
     if (key != line) continue;
-    int a = 0, b = 1;
-    if (sscanf(tab + 1, "%d\t%d", &a, &b) >= 1 && a >= 1 && a <= 8 && (b == 1 || b == 2)) {
-      *wpc = a;
-      *tile = b;
-      found = true;
-    }
+    const char* v = tab + 1;
+    Shape c{strncmp(v, "team\t", 5) == 0, 0, 1};
+    if (c.team) v += 5;
+    if (sscanf(v, "%d\t%d", &c.wpc, &c.tile) < 1) continue;
+    if (c.wpc < 1 || c.wpc > (c.team ? kTeamMaxPerCta : 8) || (c.tile != 1 && c.tile != 2)) continue;
+    *out = c;
+    found = true;
   }
   fclose(f);
   return found;
 }
-void tune_cache_store(const std::string& key, int wpc, int tile) {
+void tune_cache_store(const std::string& key, const Shape& c) {
   const char* path = getenv("SGNS_TUNE_CACHE");
   if (!path || !*path) return;
   if (FILE* f = fopen(path, "a")) {
-    fprintf(f, "%s\t%d\t%d\n", key.c_str(), wpc, tile);
+    fprintf(f, "%s\t%s%d\t%d\n", key.c_str(), c.team ? "team\t" : "", c.wpc, c.tile);
     fclose(f);
   }
 }
 
-// The forward tile used when none is given and nothing is tuned: two lanes per input for
-// fp32 tables (measured faster there), one for bf16.
-int default_tile(const sgns_handle* h) {
-  if (!window_engine_has_tile2(h->opt.size, h->opt.negative)) return 1;
-  if (h->opt.forward_tile > 0) return h->opt.forward_tile;
-  return h->opt.storage == SGNS_STORE_FP32 ? 2 : 1;
+// Teams train the workers unless the options ask for what only the one-warp kernel does: a
+// forward tile, the loss, one walk per step.
+bool teams_allowed(const sgns_options& o) { return o.forward_tile == 0 && !o.compute_loss && o.windows_per_step != 1; }
+
+// The forward tile reported when none is given.
+int default_tile(const sgns_handle* h) { return h->opt.forward_tile > 0 ? h->opt.forward_tile : 1; }
+
+// The engine of a given CTA shape (sets team and tile): a team per worker where wpc of them
+// fit a CTA, else one warp per worker.
+void shape_for_wpc(sgns_handle* h, int wpc) {
+  h->tile = default_tile(h);
+  int resident = 0;
+  h->team = teams_allowed(h->opt) && wpc <= kTeamMaxPerCta;
+  if (h->team && persistent_shape(h, wpc, &resident) != SGNS_OK) h->team = false;
 }
 
-// Autotuner: times each launch shape of the persistent engine -- warps per CTA (1..8) and,
-// where the shape has it, the forward tile (1 or 2 lanes per input) -- on a prefix of the
-// corpus, on scratch copies of the tables, and keeps the fastest (pairs per second).
+// Autotuner: times launch shapes of the persistent engine on a prefix of the corpus, on
+// scratch copies of the tables, and keeps the fastest (pairs per second).  Where teams may
+// train the workers: a team per worker at 1, 2 and 3 workers per CTA (few workers spread best
+// in small CTAs) and one warp per worker at 4..8 (the shapes that fill an SM); else one warp
+// per worker at 1..8.
 // Autotuner cache: with SGNS_TUNE_CACHE naming a file, the choice is kept per device model
 // and problem shape and reused by later runs.  The file is only an optimisation: any error
 // reading or writing it is ignored.
 sgns_status autotune(sgns_handle* h) {
   const sgns_options& o = h->opt;
   const std::string key = tune_key(h);
-  const bool tile2 = window_engine_has_tile2(o.size, o.negative);
+  auto use = [&](const Shape& c) {
+    h->team = c.team;
+    h->tile = c.tile;
+    h->wpc = c.wpc;
+  };
   if (o.warps_per_cta <= 0) {
-    int cached = 0, ctile = 1;
-    if (tune_cache_lookup(key, &cached, &ctile)) {
-      if (!tile2) ctile = 1;
-      if (o.forward_tile > 0) ctile = o.forward_tile;
-      h->tile = ctile;
-      int workers = o.workers;
-      if (!workers && persistent_shape(h, cached, &workers) != SGNS_OK) workers = 0;
-      if (workers > 0) {
-        h->wpc = cached;
-        h->workers = workers;
+    Shape c{};
+    if (tune_cache_lookup(key, &c) && (!c.team || teams_allowed(o))) {
+      if (!window_engine_has_tile2(o.size, o.negative)) c.tile = 1;
+      if (o.forward_tile > 0) c.tile = o.forward_tile;
+      use(c);
+      int workers = 0;
+      if (persistent_shape(h, c.wpc, &workers) == SGNS_OK) {
+        h->workers = o.workers > 0 ? o.workers : workers;
         h->tuned = true;
         if (o.debug > 0)
-          fprintf(stderr, "sgns: persistent engine shape from the tuning cache: %d warps/CTA, tile %d\n", cached,
-                  ctile);
+          fprintf(stderr, "sgns: persistent engine shape from the tuning cache: %d workers/CTA, tile %d, team %d\n", c.wpc,
+                  c.tile, (int)c.team);
         return SGNS_OK;
       }
     }
   }
-  if (o.warps_per_cta > 0) {  // a given CTA shape: only the tile may be left to choose
+  if (o.warps_per_cta > 0) {  // a given CTA shape
     h->wpc = o.warps_per_cta;
-    h->tile = default_tile(h);
+    shape_for_wpc(h, h->wpc);
     h->workers = o.workers;
     if (!h->workers) {
       sgns_status st = persistent_shape(h, h->wpc, &h->workers);
@@ -570,6 +597,16 @@ sgns_status autotune(sgns_handle* h) {
     h->tuned = true;
     return SGNS_OK;
   }
+  std::vector<Shape> shapes;
+  auto consider = [&](const Shape& c) {
+    int workers = 0;
+    use(c);
+    if (persistent_shape(h, c.wpc, &workers) == SGNS_OK) shapes.push_back(c);
+  };
+  if (teams_allowed(o))
+    for (int wpc = 1; wpc <= kTeamMaxPerCta; wpc++) consider(Shape{true, wpc, 1});
+  for (int wpc = shapes.empty() ? 1 : 4; wpc <= 8; wpc++) consider(Shape{false, wpc, default_tile(h)});
+  if (shapes.empty()) return fail(h, SGNS_EINVAL, "no persistent-engine shape fits this configuration");
   // the trial launches train scratch copies of the tables; the handle's own pointers,
   // corpus length and pass count are put back on every path out of the search
   const size_t tbytes = (size_t)h->V * o.size * elem_bytes(o);
@@ -587,30 +624,28 @@ sgns_status autotune(sgns_handle* h) {
     dfree(woh_s);
   };
   double best = -1.0;
-  int best_wpc = 1, best_workers = 0, best_tile = default_tile(h);
+  Shape best_shape = shapes[0];
+  int best_workers = 0;
   sgns_status st = SGNS_OK;
   cudaError_t e;
   if ((e = cudaMalloc(&wih_s, tbytes)) != cudaSuccess || (e = cudaMalloc(&woh_s, tbytes)) != cudaSuccess) {
     // no room for scratch tables: take, untimed, the shape with the most resident
-    // workers (warps per SM bound this latency-bound kernel); ties go to the wider CTA
+    // workers; ties go to the first (teams before single warps, small CTAs before large ones)
     restore();
     cudaGetLastError();
-    h->tile = best_tile;
-    for (int wpc = 1; wpc <= 8; wpc++) {
+    for (const Shape& c : shapes) {
       int workers = 0;
-      if (persistent_shape(h, wpc, &workers) != SGNS_OK) continue;
-      if (workers >= best_workers) {
-        best_wpc = wpc;
+      use(c);
+      if (persistent_shape(h, c.wpc, &workers) == SGNS_OK && workers > best_workers) {
+        best_shape = c;
         best_workers = workers;
       }
     }
-    if (best_workers == 0) return fail(h, SGNS_EINVAL, "no persistent-engine shape fits this configuration");
-    if (o.workers > 0) best_workers = o.workers;
-    h->wpc = best_wpc;
-    h->workers = best_workers;
+    use(best_shape);
+    h->workers = o.workers > 0 ? o.workers : best_workers;
     h->tuned = true;
     if (o.debug > 0)
-      fprintf(stderr, "sgns: no memory for autotuning; persistent engine at %d warps/CTA\n", best_wpc);
+      fprintf(stderr, "sgns: no memory for autotuning; persistent engine at %d warps/CTA\n", best_shape.wpc);
     return SGNS_OK;
   }
   if ((e = cudaMemcpyAsync(wih_s, h->wih, tbytes, cudaMemcpyDeviceToDevice, h->stream)) != cudaSuccess ||
@@ -621,47 +656,40 @@ sgns_status autotune(sgns_handle* h) {
   h->wih = wih_s;
   h->woh = woh_s;
   h->opt.iter = 1;
-  const int tile_lo = o.forward_tile > 0 ? o.forward_tile : 1;
-  const int tile_hi = o.forward_tile > 0 ? o.forward_tile : (tile2 ? 2 : 1);
-  for (int tile = tile_lo; tile <= tile_hi && !st; tile++) {
-    h->tile = tile;
-    for (int wpc = 1; wpc <= 8; wpc++) {
-      int workers = 0;
-      st = persistent_shape(h, wpc, &workers);
-      if (st) {
-        st = SGNS_OK;
-        continue;
-      }
-      if (o.workers > 0) workers = o.workers;
-      // a prefix long enough to give every worker a few hundred steps
-      h->n_tokens = std::min<int64_t>(n0, (int64_t)workers * 2000);
-      float ms = 0.f;
-      st = run_persistent(h, workers, wpc, false, &ms);
-      if (st) break;
-      if ((e = cudaMemcpy(h->h_ctr, h->d_ctr, sizeof(DeviceCounters), cudaMemcpyDeviceToHost)) != cudaSuccess) {
-        st = fail(h, SGNS_ECUDA, "autotuner counters: %s", cudaGetErrorString(e));
-        break;
-      }
-      const double rate = ms > 0 ? (double)h->h_ctr->pairs / ms : 0.0;
-      if (rate > best) {
-        best = rate;
-        best_wpc = wpc;
-        best_workers = workers;
-        best_tile = tile;
-      }
+  for (const Shape& c : shapes) {
+    int workers = 0;
+    use(c);
+    st = persistent_shape(h, c.wpc, &workers);
+    if (st) break;
+    if (o.workers > 0) workers = o.workers;
+    // a prefix long enough to give every worker a few hundred steps
+    h->n_tokens = std::min<int64_t>(n0, (int64_t)workers * 2000);
+    float ms = 0.f;
+    st = run_persistent(h, workers, c.wpc, false, &ms);
+    if (st) break;
+    if ((e = cudaMemcpy(h->h_ctr, h->d_ctr, sizeof(DeviceCounters), cudaMemcpyDeviceToHost)) != cudaSuccess) {
+      st = fail(h, SGNS_ECUDA, "autotuner counters: %s", cudaGetErrorString(e));
+      break;
+    }
+    const double rate = ms > 0 ? (double)h->h_ctr->pairs / ms : 0.0;
+    if (o.debug > 2)
+      fprintf(stderr, "sgns: trial team %d, %d per CTA, tile %d: %d workers, %.3f ms, %.3f G pairs/s\n", (int)c.team, c.wpc,
+              c.tile, workers, ms, rate / 1e6);
+    if (rate > best) {
+      best = rate;
+      best_shape = c;
+      best_workers = workers;
     }
   }
   restore();
   if (st) return st;
-  if (best_workers == 0) return fail(h, SGNS_EINVAL, "no persistent-engine shape fits this configuration");
-  h->wpc = best_wpc;
+  use(best_shape);
   h->workers = best_workers;
-  h->tile = best_tile;
   h->tuned = true;
-  tune_cache_store(key, best_wpc, best_tile);
+  tune_cache_store(key, best_shape);
   if (o.debug > 0)
-    fprintf(stderr, "sgns: autotuned persistent engine: %d warps/CTA, tile %d, %d workers\n", h->wpc, h->tile,
-            h->workers);
+    fprintf(stderr, "sgns: autotuned persistent engine: team %d, %d workers/CTA, tile %d, %d workers\n", (int)h->team, h->wpc,
+            h->tile, h->workers);
   return SGNS_OK;
 }
 
@@ -1029,7 +1057,7 @@ sgns_status sgns_train(sgns_handle* h) {
     if (exact) {  // one worker in a one-warp CTA: nothing to tune
       workers = 1;
       h->wpc = h->opt.warps_per_cta > 0 ? h->opt.warps_per_cta : 1;
-      h->tile = default_tile(h);
+      shape_for_wpc(h, h->wpc);
       st = run_persistent(h, 1, h->wpc, true, &ms);
       if (st) return st;
       return finish_stats(h, workers, ms);

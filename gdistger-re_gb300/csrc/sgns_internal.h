@@ -166,9 +166,7 @@ struct TrainParams {
   float start_alpha, alpha_denom;
   uint64_t sr_seed;
   int32_t compute_loss, lmax, storage;
-  int32_t fwd_tile;                // lanes per input in the forward (1, or 2 where supported)
   int32_t windows;                 // windows per step: 2 (two walks, dsgl.hpp:1100-1132) or 1
-  int32_t pad2;
   DeviceCounters* ctr;
   // plain-engine state (HBM)
   void* plain_state;
@@ -191,11 +189,16 @@ cudaError_t launch_scatter_rows(void* tab, int storage, int d, const int32_t* ro
 cudaError_t launch_widen_bf16(const void* src, float* dst, int64_t n, cudaStream_t s);
 cudaError_t launch_max_walk(const int32_t* rows, int64_t n, int32_t* out, cudaStream_t s);
 size_t window_smem_bytes(int d, int window, int K, int lmax, int warps_per_cta);
-cudaError_t window_engine_occupancy(int storage, int d, int window, int K, int lmax, int wpc, int tile,
-                                    int* ctas_per_sm);
-// whether a problem shape has the two-lanes-per-input forward (d <= 128, K <= 5)
+cudaError_t window_engine_occupancy(int storage, int d, int window, int K, int lmax, int wpc, int* ctas_per_sm);
+// whether a problem shape takes forward_tile = 2 (d <= 128, K <= 5)
 inline bool window_engine_has_tile2(int d, int K) { return d <= 128 && K <= 5; }
 cudaError_t launch_window_engine(const TrainParams& p, int warps_per_cta, cudaStream_t s);
+// the persistent engine with a team of kTeamWarps warps (four compute, one planner) per worker;
+// at most kTeamMaxPerCta workers per CTA
+constexpr int kTeamWarps = 5, kTeamMaxPerCta = 3;
+cudaError_t team_engine_occupancy(int storage, int d, int window, int K, int lmax, int workers_per_cta,
+                                  int* ctas_per_sm);
+cudaError_t launch_team_engine(const TrainParams& p, int workers_per_cta, cudaStream_t s);
 size_t plain_worker_bytes(int d, int window, int K, int lmax);
 cudaError_t launch_plain_init(const TrainParams& p, cudaStream_t s);
 cudaError_t launch_plain_step(const TrainParams& p, cudaStream_t s);

@@ -74,16 +74,16 @@ typedef struct sgns_options {
   int32_t storage;     /* sgns_storage                                            */
   int32_t engine;      /* sgns_engine                                             */
   int32_t workers;     /* independent trainers (the reference's compute threads); 0 = tuned */
-  int32_t warps_per_cta; /* persistent engine CTA shape; 0 = tuned                */
+  int32_t warps_per_cta; /* persistent engine: workers per CTA, 1..8; 0 = tuned    */
   int32_t device;      /* CUDA device ordinal                                     */
   int32_t compute_loss;/* 1 = also accumulate the SGNS loss (fp64 reduction)      */
   int32_t mode;        /* sgns_mode (-mode hogwild|exact)                         */
   int64_t table_size;  /* unigram table entries (the reference fixes 1e8, dsgl.hpp:82) */
   uint64_t seed;       /* stochastic-rounding stream seed                         */
-  int32_t forward_tile;/* persistent engine, lanes per input row in the forward dot
-                          products: 1 = one lane per input; 2 = two lanes per input while
-                          at most 16 inputs remain (d <= 128, K <= 5 only; the same sums);
-                          0 = chosen by the autotuner                              */
+  int32_t forward_tile;/* persistent engine with one warp per worker (1, or 2 with d <= 128,
+                          K <= 5): a hint of earlier kernels.  Both values run the same
+                          register-tiled forward and the same sums; 0 = also lets a team of
+                          warps train each worker where that is faster (autotuned)         */
   int32_t windows_per_step; /* 2 (or 0): the reference's step over two walks, target 1
                           labelling walk 1's window and target 2 walk 2's (dsgl.hpp:
                           1100-1159); 1: one walk per step -- its window and target with
@@ -105,9 +105,9 @@ typedef struct sgns_stats {
   uint64_t row_loads;          /* table rows copied into worker buffers              */
   uint64_t row_stores;         /* table rows written back from worker buffers        */
   uint64_t output_rows;        /* sum over steps of the output rows (targets + negatives) */
-  int32_t forward_tile;        /* persistent engine: lanes per input in the forward      */
-  int32_t warps_per_worker;    /* warps that train one worker (one: its state lives in
-                                  that warp's registers and shared memory)              */
+  int32_t forward_tile;        /* persistent engine: the option's value, 1 when tuned    */
+  int32_t warps_per_worker;    /* warps that train one worker: 1, or 5 where a team does
+                                  (four compute warps and a planner)                    */
 } sgns_stats;
 
 /* Defaults of dsgl.hpp:67-76, table_size 1e8, persistent engine, fp32. */
