@@ -27,11 +27,23 @@
 // reduction with ln 2 split into its float head and the remainder, exp(r) by Taylor's
 // series to r^13 (Horner); tanh(x) = 1 for x >= 20.
 //
-// Kernels: one warp per directed edge for the common-neighbour counts (lanes binary-search
-// the shorter list's entries in the longer one); one thread per walker for the walks, its
-// path history in shared memory (column-major by thread, so a warp scanning position i
-// reads 32 consecutive words).  The walks run twice -- lengths, then, after an exclusive
-// scan of length + 1, the tokens at their offsets -- so no per-walk buffer is needed.
+// What bounds it: a warp's double instruction holds the SM's double unit for 16 cycles, so the
+// length pass does as few of them as the exact result allows:
+//   * the walk's vertex count is also its update count, so every division of the update is by
+//     an integer n <= 1001: a * (1/n) with a host-rounded reciprocal, corrected by its exact
+//     remainder (Markstein 1990), is the rounded quotient -- three operations;
+//   * the moments of the length alone (ES, ESS, their deviation) are a table over n;
+//   * R is needed after min_length moves only, and its test R*R < r first compares
+//     ex*ex with r DH DS and takes the square root and quotient only within 2^-40 of equality;
+//   * the trace test likewise runs in fp32 unless the draw is within 1e-4 of the threshold.
+// About 25 double operations per vertex (35 past min_length) instead of about 200.  The token
+// pass knows every walk's length and so repeats only the draws and the neighbour reads.
+//
+// Kernels: one thread per directed edge for the common-neighbour counts; one thread per
+// walker for the walks, taking its next walker as soon as one ends (lengths differ by a
+// factor of four), its path history in shared memory, four vertices to 16 bytes.  Between the
+// two passes an exclusive scan of length + 1 gives each walk's place, so no per-walk buffer
+// is needed.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -65,34 +77,29 @@ __device__ __forceinline__ double tanh_pos(double x) {
   return __ddiv_rn(__dsub_rn(E, 1.0), __dadd_rn(E, 1.0));
 }
 
-struct Corr {
-  double H, EH, ES, EHS, EHH, ESS, N, R;
-};
-
-// Correlation::iterate (walk.hpp:330-365) with step 1; S = the walk's vertex count
-__device__ __forceinline__ void corr_iterate(Corr& c, const double* __restrict__ xl, int S, int f) {
-  const double t = __dsub_rn(__dadd_rn(__dsub_rn(__ldg(&xl[S]), __ldg(&xl[S + 1])), __ldg(&xl[f + 1])), __ldg(&xl[f]));
-  const double S0 = (double)S, S1 = (double)(S + 1);
-  const double H1 = __ddiv_rn(__dsub_rn(__dmul_rn(S0, c.H), t), S1);
-  const double N1 = __dadd_rn(c.N, 1.0);
-  c.EH = __dadd_rn(c.EH, __ddiv_rn(__dsub_rn(H1, c.EH), N1));
-  c.ES = __dadd_rn(c.ES, __ddiv_rn(__dsub_rn(S1, c.ES), N1));
-  c.EHS = __dadd_rn(c.EHS, __ddiv_rn(__dsub_rn(__dmul_rn(H1, S1), c.EHS), N1));
-  c.EHH = __dadd_rn(c.EHH, __ddiv_rn(__dsub_rn(__dmul_rn(H1, H1), c.EHH), N1));
-  c.ESS = __dadd_rn(c.ESS, __ddiv_rn(__dsub_rn(__dmul_rn(S1, S1), c.ESS), N1));
-  const double DH = __dsub_rn(c.EHH, __dmul_rn(c.EH, c.EH));
-  const double DS = __dsub_rn(c.ESS, __dmul_rn(c.ES, c.ES));
-  const double ex = __dsub_rn(c.EHS, __dmul_rn(c.EH, c.ES));
-  c.R = ex == 0.0 ? 0.0 : __ddiv_rn(ex, __dsqrt_rn(__dmul_rn(DH, DS)));
-  c.H = H1;
-  c.N = N1;
+// a / n for an integer n with reciprocal r = rn(1 / n): the quotient's distance from a rounding
+// boundary is at least 1 / (2 n) of its last place, the corrected sum's error 2^-51 of it
+__device__ __forceinline__ double div_by(double a, double n, double r) {
+  const double q = __dmul_rn(a, r);
+  return __fma_rn(__fma_rn(-q, n, a), r, q);
 }
+
+// What an update to a walk of n vertices reads, whatever the walk (kWalkMaxLength + 2 entries,
+// built on the host by walk_length_table).
+static_assert(kWalkTableDoubles == 4, "LengthTable");
+struct __align__(16) LengthTable {
+  double dxl;  // (n-1) log2 (n-1) - n log2 n
+  double rcp;  // 1 / n
+  double es;   // the running mean of the length after the update
+  double ds;   // its deviation ESS - ES^2
+};
 
 struct WalkArgs {
   const int64_t* indptr;
   const int32_t* indices;
   const int32_t* cn;
-  const double* xl;
+  const double* xl;         // x log2 x
+  const LengthTable* len;
   int64_t V, walker_num;
   int32_t min_length, max_length;
   double r_threshold;
@@ -103,69 +110,167 @@ struct WalkArgs {
   int32_t* corpus;         // pass 2 output
 };
 
-// kWrite = false: lengths[w]; kWrite = true: the walk's tokens and its -1 at offsets[w].
-template <bool kWrite>
-__global__ void __launch_bounds__(256) info_walk_kernel(WalkArgs a) {
-  extern __shared__ int32_t hist_s[];  // [max_length][blockDim.x]
-  const int T = blockDim.x, tid = threadIdx.x;
-  int32_t* hist = hist_s + tid;
-  for (int64_t w = (int64_t)blockIdx.x * T + tid; w < a.walker_num; w += (int64_t)gridDim.x * T) {
-    const int64_t start = w % a.V;
-    uint64_t ctr = mix64(a.seed ^ ((uint64_t)w * kGolden));
-    int len = 1;
-    hist[0] = (int32_t)start;
-    Corr c{0.0, 0.0, 1.0, 0.0, 0.0, 1.0, 1.0, 1.0};
-    int steps = 0, redraws = 0;
-    int64_t cur = start;
-    bool done = len >= a.max_length;
-    // appends v; returns true when the walk stops there
-    auto append = [&](int32_t v) -> bool {
-      int f = 0;
-      for (int i = 0; i < len; i++) f += hist[i * T] == v;
-      corr_iterate(c, a.xl, len, f);
-      hist[len * T] = v;
-      len++;
-      steps++;
-      if (steps > a.min_length && (__dmul_rn(c.R, c.R) < a.r_threshold || c.R < 0.0)) return true;
-      return len >= a.max_length;
-    };
-    while (!done) {
-      const int64_t b = __ldg(&a.indptr[cur]);
-      const int64_t ds = __ldg(&a.indptr[cur + 1]) - b;
-      if (ds == 0) break;
-      uint64_t r = mix64(ctr);
+// Correlation state (Correlation::iterate, walk.hpp:330-365, step 1)
+struct Corr {
+  double H, EH, EHS, EHH;
+};
+__device__ __forceinline__ void corr_iterate(Corr& c, const LengthTable& t, double xf, double xf1, int n) {
+  const double S1 = (double)n, S0 = (double)(n - 1);
+  const double dt = __dsub_rn(__dadd_rn(t.dxl, xf1), xf);
+  const double H1 = div_by(__dsub_rn(__dmul_rn(S0, c.H), dt), S1, t.rcp);
+  c.EH = __dadd_rn(c.EH, div_by(__dsub_rn(H1, c.EH), S1, t.rcp));
+  c.EHS = __dadd_rn(c.EHS, div_by(__dsub_rn(__dmul_rn(H1, S1), c.EHS), S1, t.rcp));
+  c.EHH = __dadd_rn(c.EHH, div_by(__dsub_rn(__dmul_rn(H1, H1), c.EHH), S1, t.rcp));
+  c.H = H1;
+}
+// R*R < threshold or R < 0 (walk.hpp:868-874), R = ex / sqrt(DH DS)
+__device__ __forceinline__ bool corr_stops(const Corr& c, const LengthTable& t, double threshold) {
+  const double DH = __dsub_rn(c.EHH, __dmul_rn(c.EH, c.EH));
+  const double ex = __dsub_rn(c.EHS, __dmul_rn(c.EH, t.es));
+  const double P = __dmul_rn(DH, t.ds);
+  // clear of the boundary, of zeros and of the range's ends: the rounded R*R and ex*ex / P
+  // differ by a few last places
+  if (ex > 1e-100 && ex < 1e100 && P > 1e-100 && P < 1e100 && threshold > 1e-6 && threshold < 1e6) {
+    const double a = ex * ex, b = threshold * P, slack = b * 0x1p-40;
+    if (a < b - slack) return true;
+    if (a > b + slack) return false;
+  }
+  const double R = ex == 0.0 ? 0.0 : __ddiv_rn(ex, __dsqrt_rn(P));
+  return __dmul_rn(R, R) < threshold || R < 0.0;
+}
+// tanh(((1 / (ds - cn)) max(ds, du)) / min(ds, du)) <= p (walk.hpp:920-1031)
+__device__ __forceinline__ bool trace_step(int64_t ds, int64_t du, int32_t cn, uint64_t r) {
+  const int64_t mx = ds > du ? ds : du, mn = ds < du ? ds : du, left = ds - cn;
+  if (left > 0 && mn > 0) {
+    const float x = (float)mx / ((float)left * (float)mn);
+    const float e = __expf(2.f * fminf(x, 20.f));
+    const float th = __fdividef(e - 1.f, e + 1.f), p = (float)(r >> 40) * 0x1p-24f;
+    if (fabsf(th - p) > 1e-4f) return th < p;
+  }
+  const double p = __dmul_rn((double)(r >> 11), 1.0 / 9007199254740992.0);
+  const double pa = __ddiv_rn(__dmul_rn(__ddiv_rn(1.0, (double)left), (double)mx), (double)mn);
+  return tanh_pos(pa) <= p;
+}
+
+// A walker's draws and moves; both passes make the same ones.
+struct Walker {
+  int64_t cur;
+  uint64_t ctr;
+  __device__ __forceinline__ void start(const WalkArgs& a, int64_t w) {
+    cur = w % a.V;
+    ctr = mix64(a.seed ^ ((uint64_t)w * kGolden));
+  }
+  // The next candidate: false when the walk ends here.  moved: no longer at the walk's first
+  // vertex (before that a candidate equal to it is drawn again).
+  __device__ __forceinline__ bool candidate(const WalkArgs& a, bool moved, int32_t* u, bool* trace) {
+    const int64_t b = __ldg(&a.indptr[cur]);
+    const int64_t ds = __ldg(&a.indptr[cur + 1]) - b;
+    if (ds == 0) return false;
+    int64_t e = 0;
+    for (int redraws = 0;; redraws++) {
+      const uint64_t r = mix64(ctr);
       ctr += kGolden;
-      const int64_t e = b + (int64_t)(((r >> 32) * (uint64_t)ds) >> 32);
-      const int32_t u = __ldg(&a.indices[e]);
-      if (ds == 2 && __ldg(&a.indices[b]) == cur) break;
-      if (steps == 0 && u == cur) {
-        if (++redraws >= kMaxRedraws) break;
-        continue;
-      }
-      bool trace = false;
-      if (a.trace) {
-        r = mix64(ctr);
-        ctr += kGolden;
-        const double p = __dmul_rn((double)(r >> 11), 1.0 / 9007199254740992.0);
-        const int64_t du = __ldg(&a.indptr[(int64_t)u + 1]) - __ldg(&a.indptr[u]);
-        const int64_t mx = ds > du ? ds : du, mn = ds < du ? ds : du;
-        const double pa =
-            __ddiv_rn(__dmul_rn(__ddiv_rn(1.0, (double)(ds - __ldg(&a.cn[e]))), (double)mx), (double)mn);
-        trace = tanh_pos(pa) <= p;
-      }
-      if (append(u)) break;
-      if (trace) {
-        if (append((int32_t)cur)) break;
-      } else {
-        cur = u;
-      }
+      e = b + (int64_t)(((r >> 32) * (uint64_t)ds) >> 32);
+      *u = __ldg(&a.indices[e]);
+      if (ds == 2 && __ldg(&a.indices[b]) == cur) return false;
+      if (moved || *u != cur) break;
+      if (redraws + 1 >= kMaxRedraws) return false;
     }
-    if (!kWrite) {
+    *trace = false;
+    if (a.trace) {
+      const uint64_t r = mix64(ctr);
+      ctr += kGolden;
+      const int64_t du = __ldg(&a.indptr[(int64_t)*u + 1]) - __ldg(&a.indptr[*u]);
+      *trace = trace_step(ds, du, __ldg(&a.cn[e]), r);
+    }
+    return true;
+  }
+};
+
+// Pass 1: lengths[w].  Shared memory: the tables' first max_length + 2 entries, then the path
+// histories, four vertices to an int4, [ceil(max_length / 4)][blockDim.x].
+__global__ void __launch_bounds__(256) walk_lengths_kernel(WalkArgs a) {
+  extern __shared__ __align__(16) unsigned char walk_smem[];
+  const int T = blockDim.x, tid = threadIdx.x, entries = a.max_length + 2;
+  LengthTable* tab = reinterpret_cast<LengthTable*>(walk_smem);
+  double* xl = reinterpret_cast<double*>(tab + entries);
+  int4* hist = reinterpret_cast<int4*>(xl + ((entries + 1) & ~1)) + tid;
+  for (int i = tid; i < entries; i += T) {
+    tab[i] = a.len[i];
+    xl[i] = a.xl[i];
+  }
+  __syncthreads();
+  const int64_t stride = (int64_t)gridDim.x * T;
+  int64_t w = (int64_t)blockIdx.x * T + tid;
+  Walker k{};
+  Corr c{};
+  int len = 0;
+  auto begin = [&]() {
+    k.start(a, w);
+    c = Corr{0.0, 0.0, 0.0, 0.0};
+    hist[0] = make_int4((int32_t)k.cur, -1, -1, -1);
+    len = 1;
+  };
+  // appends v; true when the walk stops there
+  auto append = [&](int32_t v) -> bool {
+    int f = 0;
+    for (int g = 0; 4 * g < len; g++) {
+      const int4 h = hist[g * T];
+      f += (h.x == v) + (h.y == v) + (h.z == v) + (h.w == v);
+    }
+    if ((len & 3) == 0) hist[(len >> 2) * T] = make_int4(v, -1, -1, -1);
+    else reinterpret_cast<int32_t*>(&hist[(len >> 2) * T])[len & 3] = v;
+    len++;
+    const LengthTable t = tab[len];
+    corr_iterate(c, t, xl[f], xl[f + 1], len);
+    // len - 1 vertices appended so far
+    if (len - 1 > a.min_length && corr_stops(c, t, a.r_threshold)) return true;
+    return len >= a.max_length;
+  };
+  if (w < a.walker_num) begin();
+  while (w < a.walker_num) {
+    int32_t u;
+    bool trace, done = len >= a.max_length || !k.candidate(a, len > 1, &u, &trace);
+    if (!done) {
+      done = append(u);
+      if (!trace) k.cur = u;
+      else if (!done) done = append((int32_t)k.cur);
+    }
+    if (done) {
       a.lengths[w] = len;
+      w += stride;
+      if (w < a.walker_num) begin();
+    }
+  }
+}
+
+// Pass 2: the walk's tokens and its -1 at offsets[w].
+__global__ void __launch_bounds__(256) walk_tokens_kernel(WalkArgs a) {
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  Walker k{};
+  int32_t *out = nullptr, *last = nullptr;  // next token, place of the -1
+  bool moved = false;
+  auto begin = [&]() {
+    k.start(a, w);
+    out = a.corpus + a.offsets[w];
+    last = a.corpus + a.offsets[w + 1] - 1;
+    *out++ = (int32_t)k.cur;
+    moved = false;
+  };
+  if (w < a.walker_num) begin();
+  while (w < a.walker_num) {
+    int32_t u;
+    bool trace;
+    if (out < last && k.candidate(a, moved, &u, &trace)) {
+      moved = true;
+      *out++ = u;
+      if (!trace) k.cur = u;
+      else if (out < last) *out++ = (int32_t)k.cur;
     } else {
-      int32_t* out = a.corpus + a.offsets[w];
-      for (int i = 0; i < len; i++) out[i] = hist[i * T];
-      out[len] = -1;
+      *out = -1;
+      w += stride;
+      if (w < a.walker_num) begin();
     }
   }
 }
@@ -231,47 +336,78 @@ __global__ void add_tile_offsets_kernel(int64_t* offsets, int64_t n, const int64
 }
 
 // ---- common-neighbour counts ----------------------------------------------------------
-// One warp per directed edge e = (u, v): u is found by binary search in indptr; lanes take
-// entries of the shorter adjacency list and binary-search them in the longer one.
+// One thread per directed edge e = (u, v).  A block takes tiles of consecutive edges: the
+// sources of a tile's first and last edge are found in indptr once, every other source between
+// them.  The entries of the shorter adjacency list are searched in the longer one: by the
+// thread itself up to kOwnEntries of them, else by the whole warp, edge after edge.
 // status bits: 1 = a neighbour outside [0, V), 2 = an adjacency list not strictly increasing.
-__global__ void __launch_bounds__(256) edge_cn_kernel(const int64_t* __restrict__ indptr,
-                                                      const int32_t* __restrict__ indices, int64_t V, int64_t E,
-                                                      int32_t* __restrict__ cn, int32_t* status) {
+constexpr int kEdgeTile = 256, kOwnEntries = 24;
+
+// the largest u in [lo, hi) with indptr[u] <= e
+__device__ __forceinline__ int64_t source_of(const int64_t* __restrict__ indptr, int64_t e, int64_t lo, int64_t hi) {
+  while (hi - lo > 1) {
+    const int64_t mid = (lo + hi) >> 1;
+    if (__ldg(&indptr[mid]) <= e) lo = mid;
+    else hi = mid;
+  }
+  return lo;
+}
+// entries [i, se) by `step` of the shorter list that the sorted list [lb, le) holds
+__device__ __forceinline__ int count_in(const int32_t* __restrict__ indices, int64_t i, int64_t se, int step, int64_t lb,
+                                        int64_t le) {
+  int c = 0;
+  for (; i < se; i += step) {
+    const int32_t x = __ldg(&indices[i]);
+    int64_t l = lb, h = le;  // first position with indices >= x
+    while (l < h) {
+      const int64_t m = (l + h) >> 1;
+      if (__ldg(&indices[m]) < x) l = m + 1;
+      else h = m;
+    }
+    c += (l < le && __ldg(&indices[l]) == x);
+  }
+  return c;
+}
+__global__ void __launch_bounds__(kEdgeTile) edge_cn_kernel(const int64_t* __restrict__ indptr,
+                                                            const int32_t* __restrict__ indices, int64_t V, int64_t E,
+                                                            int32_t* __restrict__ cn, int32_t* status) {
+  __shared__ int64_t range[2];
   const int lane = threadIdx.x & 31;
-  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  for (int64_t e = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; e < E; e += warps) {
-    int64_t lo = 0, hi = V;  // the largest u with indptr[u] <= e
-    while (hi - lo > 1) {
-      const int64_t mid = (lo + hi) >> 1;
-      if (__ldg(&indptr[mid]) <= e) lo = mid;
-      else hi = mid;
+  for (int64_t base = (int64_t)blockIdx.x * kEdgeTile; base < E; base += (int64_t)gridDim.x * kEdgeTile) {
+    __syncthreads();
+    if (threadIdx.x < 2) {
+      const int64_t last = base + kEdgeTile < E ? base + kEdgeTile - 1 : E - 1;
+      range[threadIdx.x] = source_of(indptr, threadIdx.x ? last : base, 0, V);
     }
-    const int64_t u = lo;
-    const int32_t v = __ldg(&indices[e]);
-    const int64_t ub = __ldg(&indptr[u]), ue = __ldg(&indptr[u + 1]);
-    if (v < 0 || v >= V) {
-      if (lane == 0) atomicOr(status, 1);
-      if (lane == 0) cn[e] = 0;
-      continue;
-    }
-    if (lane == 0 && e > ub && __ldg(&indices[e - 1]) >= v) atomicOr(status, 2);
-    const int64_t vb = __ldg(&indptr[v]), ve = __ldg(&indptr[v + 1]);
-    const bool u_short = ue - ub <= ve - vb;
-    const int64_t sb = u_short ? ub : vb, se = u_short ? ue : ve;
-    const int64_t lb = u_short ? vb : ub, le = u_short ? ve : ue;
-    int c = 0;
-    for (int64_t i = sb + lane; i < se; i += 32) {
-      const int32_t x = __ldg(&indices[i]);
-      int64_t l = lb, h = le;  // first position with indices >= x
-      while (l < h) {
-        const int64_t m = (l + h) >> 1;
-        if (__ldg(&indices[m]) < x) l = m + 1;
-        else h = m;
+    __syncthreads();
+    const int64_t e = base + threadIdx.x;
+    int64_t sb = 0, se = 0, lb = 0, le = 0;
+    if (e < E) {
+      const int64_t u = source_of(indptr, e, range[0], range[1] + 1);
+      const int32_t v = __ldg(&indices[e]);
+      if (v < 0 || v >= V) {
+        atomicOr(status, 1);
+      } else {
+        const int64_t ub = __ldg(&indptr[u]), ue = __ldg(&indptr[u + 1]);
+        if (e > ub && __ldg(&indices[e - 1]) >= v) atomicOr(status, 2);
+        const int64_t vb = __ldg(&indptr[v]), ve = __ldg(&indptr[v + 1]);
+        const bool u_short = ue - ub <= ve - vb;
+        sb = u_short ? ub : vb, se = u_short ? ue : ve;
+        lb = u_short ? vb : ub, le = u_short ? ve : ue;
       }
-      c += (l < le && __ldg(&indices[l]) == x);
     }
-    c = __reduce_add_sync(0xFFFFFFFFu, c);
-    if (lane == 0) cn[e] = c;
+    const bool own = se - sb <= kOwnEntries;
+    int c = own ? count_in(indices, sb, se, 1, lb, le) : 0;
+    unsigned rest = __ballot_sync(0xFFFFFFFFu, !own);
+    while (rest) {
+      const int k = __ffs(rest) - 1;
+      rest &= rest - 1;
+      const int64_t b = __shfl_sync(0xFFFFFFFFu, sb, k), n = __shfl_sync(0xFFFFFFFFu, se, k);
+      const int64_t l0 = __shfl_sync(0xFFFFFFFFu, lb, k), l1 = __shfl_sync(0xFFFFFFFFu, le, k);
+      const int t = __reduce_add_sync(0xFFFFFFFFu, count_in(indices, b + lane, n, 32, l0, l1));
+      if (lane == k) c = t;
+    }
+    if (e < E) cn[e] = c;
   }
 }
 
@@ -303,11 +439,24 @@ cudaError_t launch_validate_csr(const int64_t* indptr, const int32_t* indices, i
   return cudaGetLastError();
 }
 
-int walk_block_threads(int max_length) {
-  // history words per thread: max_length; at most 96 KB of shared memory per block
-  int t = (96 * 1024) / (4 * max_length);
-  t = t >= 256 ? 256 : (t / 32) * 32;
-  return t < 32 ? 32 : t;
+static size_t walk_table_smem(int max_length) {
+  const size_t entries = (size_t)max_length + 2;
+  return entries * sizeof(LengthTable) + ((entries + 1) & ~(size_t)1) * sizeof(double);
+}
+static size_t walk_smem(int max_length, int threads) {
+  return walk_table_smem(max_length) + sizeof(int4) * (size_t)((max_length + 3) / 4) * threads;
+}
+// Threads per block of the length pass: the most walkers resident on an SM (228 KB of shared
+// memory, 1 KB reserved per block), the larger block on a tie.
+static int walk_block_threads(int max_length) {
+  int best = 32, resident = 0;
+  for (int t = 32; t <= 256; t += 32) {
+    const size_t smem = walk_smem(max_length, t);
+    if (smem > 232448) break;
+    const int r = (int)(233472 / (smem + 1024)) * t;
+    if (r >= resident) best = t, resident = r;
+  }
+  return best;
 }
 
 size_t walk_scratch_bytes(int64_t walker_num) {
@@ -319,9 +468,9 @@ size_t walk_scratch_bytes(int64_t walker_num) {
 // Pass 1 (lengths) and the scan; *offsets_out points into scratch (walker_num + 1 entries,
 // the last = total tokens).
 cudaError_t launch_info_walks_count(const int64_t* indptr, const int32_t* indices, const int32_t* cn,
-                                    const double* xl, int64_t V, int64_t walker_num, int min_length,
-                                    int max_length, double r_threshold, uint64_t seed, int trace, void* scratch,
-                                    int num_sms, int64_t** offsets_out, cudaStream_t s) {
+                                    const double* xl, const double* len_table, int64_t V, int64_t walker_num,
+                                    int min_length, int max_length, double r_threshold, uint64_t seed, int trace,
+                                    void* scratch, int num_sms, int64_t** offsets_out, cudaStream_t s) {
   char* p = static_cast<char*>(scratch);
   int64_t* offsets = reinterpret_cast<int64_t*>(p);
   p += sizeof(int64_t) * (size_t)(walker_num + 1);
@@ -329,21 +478,18 @@ cudaError_t launch_info_walks_count(const int64_t* indptr, const int32_t* indice
   int64_t* tile_sums = reinterpret_cast<int64_t*>(p);
   p += sizeof(int64_t) * (size_t)(tiles + 1);
   int32_t* lengths = reinterpret_cast<int32_t*>(p);
-  WalkArgs a{indptr, indices, cn, xl, V, walker_num, min_length, max_length, r_threshold, seed, trace, lengths,
-             nullptr, nullptr};
+  const WalkArgs a{indptr, indices, cn, xl, reinterpret_cast<const LengthTable*>(len_table), V, walker_num, min_length,
+                   max_length, r_threshold, seed, trace, lengths, nullptr, nullptr};
   const int T = walk_block_threads(max_length);
-  const size_t smem = sizeof(int32_t) * (size_t)T * max_length;
-  cudaError_t e = cudaFuncSetAttribute(info_walk_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(info_walk_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const size_t smem = walk_smem(max_length, T);
+  cudaError_t e = cudaFuncSetAttribute(walk_lengths_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, info_walk_kernel<false>, T, smem);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, walk_lengths_kernel, T, smem);
   if (e != cudaSuccess) return e;
   const int64_t want = (walker_num + T - 1) / T;
-  const int64_t resident = (int64_t)num_sms * (per_sm > 0 ? per_sm : 1);
-  const unsigned grid = (unsigned)(want < resident * 8 ? want : resident * 8);
-  info_walk_kernel<false><<<grid, T, smem, s>>>(a);
+  const int64_t resident = (int64_t)num_sms * (per_sm > 0 ? per_sm : 1);  // threads take walkers in turn
+  walk_lengths_kernel<<<(unsigned)(want < resident ? want : resident), T, smem, s>>>(a);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   scan_tiles_kernel<<<(unsigned)tiles, kScanBlock, 0, s>>>(lengths, walker_num, offsets, tile_sums);
   scan_tile_sums_kernel<<<1, kScanBlock, 0, s>>>(tile_sums, tiles);
@@ -353,30 +499,23 @@ cudaError_t launch_info_walks_count(const int64_t* indptr, const int32_t* indice
 }
 
 // Pass 2: the walks again, written at their offsets.
-cudaError_t launch_info_walks_emit(const int64_t* indptr, const int32_t* indices, const int32_t* cn,
-                                   const double* xl, int64_t V, int64_t walker_num, int min_length, int max_length,
-                                   double r_threshold, uint64_t seed, int trace, const int64_t* offsets,
+cudaError_t launch_info_walks_emit(const int64_t* indptr, const int32_t* indices, const int32_t* cn, int64_t V,
+                                   int64_t walker_num, uint64_t seed, int trace, const int64_t* offsets,
                                    int32_t* corpus, int num_sms, cudaStream_t s) {
-  WalkArgs a{indptr, indices, cn, xl, V, walker_num, min_length, max_length, r_threshold, seed, trace, nullptr,
-             offsets, corpus};
-  const int T = walk_block_threads(max_length);
-  const size_t smem = sizeof(int32_t) * (size_t)T * max_length;
-  int per_sm = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, info_walk_kernel<true>, T, smem);
-  if (e != cudaSuccess) return e;
-  const int64_t want = (walker_num + T - 1) / T;
-  const int64_t resident = (int64_t)num_sms * (per_sm > 0 ? per_sm : 1);
-  const unsigned grid = (unsigned)(want < resident * 8 ? want : resident * 8);
-  info_walk_kernel<true><<<grid, T, smem, s>>>(a);
+  WalkArgs a{};
+  a.indptr = indptr, a.indices = indices, a.cn = cn, a.V = V, a.walker_num = walker_num;
+  a.seed = seed, a.trace = trace, a.offsets = offsets, a.corpus = corpus;
+  const int64_t want = (walker_num + 255) / 256, resident = (int64_t)num_sms * 8;
+  walk_tokens_kernel<<<(unsigned)(want < resident ? want : resident), 256, 0, s>>>(a);
   return cudaGetLastError();
 }
 
 cudaError_t launch_edge_common_neighbors(const int64_t* indptr, const int32_t* indices, int64_t V, int64_t E,
                                          int32_t* cn, int32_t* status, int num_sms, cudaStream_t s) {
   if (E == 0) return cudaSuccess;
-  const int64_t want = (E * 32 + 255) / 256;
+  const int64_t want = (E + kEdgeTile - 1) / kEdgeTile;
   const int64_t cap = (int64_t)num_sms * 64;
-  edge_cn_kernel<<<(unsigned)(want < cap ? want : cap), 256, 0, s>>>(indptr, indices, V, E, cn, status);
+  edge_cn_kernel<<<(unsigned)(want < cap ? want : cap), kEdgeTile, 0, s>>>(indptr, indices, V, E, cn, status);
   return cudaGetLastError();
 }
 

@@ -272,6 +272,25 @@ void xlog2x_table(int n, double* t) {
   }
 }
 
+// What the walker's correlation update to n vertices takes, whatever the walk (Correlation::
+// iterate, walk.hpp:330-365): (n-1) log2 (n-1) - n log2 n, 1 / n, the running mean of the
+// length and its deviation ESS - ES^2, from the same operations the update would make.
+void walk_length_table(int entries, const double* xl, double* t) {
+  double es = 1.0, ess = 1.0;
+  for (int n = 0; n < entries; n++, t += kWalkTableDoubles) {
+    t[0] = t[1] = t[3] = 0.0;
+    t[2] = 1.0;
+    if (n < 2) continue;
+    const double S1 = (double)n;
+    es = es + (S1 - es) / S1;
+    ess = ess + (S1 * S1 - ess) / S1;
+    t[0] = xl[n - 1] - xl[n];
+    t[1] = 1.0 / S1;
+    t[2] = es;
+    t[3] = ess - es * es;
+  }
+}
+
 void build_exp_table(float* t) {  // dsgl.hpp:1557-1562
   for (int i = 0; i < kExpTableSize + 1; i++) {
     const float e = expf(((float)i / (float)kExpTableSize * 2 - 1) * kMaxExp);
@@ -1562,23 +1581,26 @@ sgns_status sgns_info_walks(const sgns_walk_options* o, const int64_t* indptr, c
   if (!ds) return fail(nullptr, SGNS_ECUDA, "no current CUDA device");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   std::lock_guard<std::mutex> g(ds->mx);
-  const size_t xl_bytes = sizeof(double) * (size_t)(kWalkMaxLength + 2);
-  sgns_status st = ds->ensure(256 + xl_bytes + walk_scratch_bytes(o->walker_num));
+  // x log2 x, then the per-length constants of the update
+  constexpr int kEntries = kWalkMaxLength + 2;
+  const size_t xl_bytes = sizeof(double) * (size_t)kEntries, tab_bytes = xl_bytes * (1 + kWalkTableDoubles);
+  sgns_status st = ds->ensure(256 + tab_bytes + walk_scratch_bytes(o->walker_num));
   if (st) return st;
   char* base = static_cast<char*>(ds->buf);
   int32_t* status = reinterpret_cast<int32_t*>(base);
   double* xl = reinterpret_cast<double*>(base + 256);
-  void* scratch = base + 256 + xl_bytes;
+  void* scratch = base + 256 + tab_bytes;
   if ((st = check_csr("walks", indptr, indices, V, n_edges, status, sms, s))) return st;
-  std::vector<double> hxl(kWalkMaxLength + 2);
-  xlog2x_table(kWalkMaxLength + 2, hxl.data());
+  std::vector<double> tables(tab_bytes / sizeof(double));
+  xlog2x_table(kEntries, tables.data());
+  walk_length_table(kEntries, tables.data(), tables.data() + kEntries);
   int64_t* offsets = nullptr;
   int64_t total = 0;
   cudaError_t e;
-  if ((e = cudaMemcpyAsync(xl, hxl.data(), xl_bytes, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
-      (e = launch_info_walks_count(indptr, indices, cn, xl, V, o->walker_num, o->min_length, o->max_length,
-                                   o->r_threshold, o->seed, o->trace_steps, scratch, sms, &offsets, s)) !=
-          cudaSuccess ||
+  if ((e = cudaMemcpyAsync(xl, tables.data(), tab_bytes, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
+      (e = launch_info_walks_count(indptr, indices, cn, xl, xl + kEntries, V, o->walker_num, o->min_length,
+                                   o->max_length, o->r_threshold, o->seed, o->trace_steps, scratch, sms, &offsets,
+                                   s)) != cudaSuccess ||
       (e = cudaMemcpyAsync(&total, offsets + o->walker_num, sizeof total, cudaMemcpyDeviceToHost, s)) !=
           cudaSuccess ||
       (e = cudaStreamSynchronize(s)) != cudaSuccess)
@@ -1588,8 +1610,8 @@ sgns_status sgns_info_walks(const sgns_walk_options* o, const int64_t* indptr, c
     if (cap == 0 && !corpus) return SGNS_OK;
     return fail(nullptr, SGNS_EINVAL, "walks yield %lld tokens, capacity %lld", (long long)total, (long long)cap);
   }
-  if ((e = launch_info_walks_emit(indptr, indices, cn, xl, V, o->walker_num, o->min_length, o->max_length,
-                                  o->r_threshold, o->seed, o->trace_steps, offsets, corpus, sms, s)) != cudaSuccess ||
+  if ((e = launch_info_walks_emit(indptr, indices, cn, V, o->walker_num, o->seed, o->trace_steps, offsets, corpus, sms,
+                                  s)) != cudaSuccess ||
       (e = cudaStreamSynchronize(s)) != cudaSuccess)
     return fail(nullptr, SGNS_ECUDA, "walks: %s", cudaGetErrorString(e));
   return SGNS_OK;

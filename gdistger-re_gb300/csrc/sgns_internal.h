@@ -235,15 +235,15 @@ cudaError_t launch_validate_csr(const int64_t* indptr, const int32_t* indices, i
                                 int32_t* status, int num_sms, cudaStream_t s);
 cudaError_t launch_edge_common_neighbors(const int64_t* indptr, const int32_t* indices, int64_t V, int64_t E,
                                          int32_t* cn, int32_t* status, int num_sms, cudaStream_t s);
-int walk_block_threads(int max_length);
 size_t walk_scratch_bytes(int64_t walker_num);
+// per-length constants of the walker's update, kWalkTableDoubles per length (sgns_host.cpp)
+constexpr int kWalkTableDoubles = 4;
 cudaError_t launch_info_walks_count(const int64_t* indptr, const int32_t* indices, const int32_t* cn,
-                                    const double* xl, int64_t V, int64_t walker_num, int min_length,
-                                    int max_length, double r_threshold, uint64_t seed, int trace, void* scratch,
-                                    int num_sms, int64_t** offsets_out, cudaStream_t s);
-cudaError_t launch_info_walks_emit(const int64_t* indptr, const int32_t* indices, const int32_t* cn,
-                                   const double* xl, int64_t V, int64_t walker_num, int min_length, int max_length,
-                                   double r_threshold, uint64_t seed, int trace, const int64_t* offsets,
+                                    const double* xl, const double* len_table, int64_t V, int64_t walker_num,
+                                    int min_length, int max_length, double r_threshold, uint64_t seed, int trace,
+                                    void* scratch, int num_sms, int64_t** offsets_out, cudaStream_t s);
+cudaError_t launch_info_walks_emit(const int64_t* indptr, const int32_t* indices, const int32_t* cn, int64_t V,
+                                   int64_t walker_num, uint64_t seed, int trace, const int64_t* offsets,
                                    int32_t* corpus, int num_sms, cudaStream_t s);
 
 void host_exp_table(float* t /* kExpTableSize + 1 */);
