@@ -59,89 +59,138 @@ __global__ void map_corpus_kernel(const int32_t* ids, const int32_t* row_of, int
 }
 
 // ---- explicit-row minibatch update (the step arithmetic of both trainers) ----------
+// One block of four warps per minibatch, its rows staged in shared memory.  The sums are those
+// of forward_gradient and backward (dsgl_device.cuh), one chain each, so they are spread by
+// chain: dot products by (two outputs, input), outputMd by output, updates by input.
+// What bounds it: the chains' latency (a dot product is d dependent multiply-adds) at the five
+// blocks that 43 KB of rows (64 inputs, d = 128) leave per SM.  20,000 minibatches of 19.6
+// inputs, d = 128, rounded write-back: 2,260 us with one warp per minibatch, the sigmoid table
+// copied to shared memory per block and a one-thread prefix of the counts; 142 us now.
+constexpr int kMbThreads = 128;
+constexpr int kMbOwnPrefix = 1024;  // up to here a block sums the counts before its own itself
+
+// sum over the block of each thread's a and b (int64)
+__device__ __forceinline__ void block_sum2(int64_t& a, int64_t& b, int64_t* scratch) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    a += __shfl_xor_sync(kFull, a, o);
+    b += __shfl_xor_sync(kFull, b, o);
+  }
+  if (lane_id() == 0) {
+    scratch[2 * (threadIdx.x >> 5)] = a;
+    scratch[2 * (threadIdx.x >> 5) + 1] = b;
+  }
+  __syncthreads();
+  a = b = 0;
+#pragma unroll
+  for (int k = 0; k < kMbThreads / 32; k++) {
+    a += scratch[2 * k];
+    b += scratch[2 * k + 1];
+  }
+}
+
 // kRound: instead of the updates, write each updated row (row + update) as bf16 bits with
 // the trainers' stochastic rounding (RowIO<STORE_BF16>::store4), event keys from sr_seed
-// and the minibatch index; d_in / d_out then point to uint16 rows.
-template <int DCH, bool kRound = false>
-__global__ void __launch_bounds__(32) minibatch_kernel(int d, int imax, int omax, const int32_t* in_count,
-                                                       const int32_t* in_first, const int32_t* out_count,
-                                                       const int32_t* out_meta_all, const float* alpha,
-                                                       const int64_t* in_off, const int64_t* out_off,
-                                                       const float* in_rows, const float* out_rows,
-                                                       float* d_in, float* d_out, const float* exp_table,
-                                                       int32_t* status, uint64_t sr_seed = 0) {
+// and the minibatch index; d_in / d_out then point to uint16 rows.  in_off null: the block
+// sums the counts of the minibatches before it.
+template <bool kRound>
+__global__ void __launch_bounds__(kMbThreads) minibatch_kernel(int d, int imax, int omax, const int32_t* in_count,
+                                                               const int32_t* in_first, const int32_t* out_count,
+                                                               const int32_t* out_meta_all, const float* alpha,
+                                                               const int64_t* in_off, const int64_t* out_off,
+                                                               const float* in_rows, const float* out_rows,
+                                                               float* d_in, float* d_out,
+                                                               const float* __restrict__ exp_table, int32_t* status,
+                                                               uint64_t sr_seed) {
   extern __shared__ __align__(16) float smem[];
-  const int b = blockIdx.x, lane = lane_id();
+  __shared__ int64_t sums[2 * (kMbThreads / 32)];
+  const int b = blockIdx.x, lane = lane_id(), warp = threadIdx.x >> 5;
   const int I = in_count[b], first = in_first[b], O = out_count[b];
   if (I < 1 || I > imax || O < 2 || O > omax || first < 0 || first > I) {
-    if (lane == 0) atomicExch(status, 1);
+    if (threadIdx.x == 0) atomicExch(status, 1);
     return;
   }
-  const int DP = d + 4;
-  float* exp_s = smem;
-  float* xin = smem + 1004;
-  float* outI = xin + (size_t)imax * DP;
-  float2* corrP = reinterpret_cast<float2*>(outI + (size_t)kOMax * d);
-  int* meta = reinterpret_cast<int*>(corrP + (size_t)imax * (kOMax + 2));
-  for (int i = lane; i < kExpTableSize + 1; i += 32) exp_s[i] = exp_table[i];
-  const int d4 = d >> 2;
-  const float* gin = in_rows + in_off[b] * d;
-  const float* gout = out_rows + out_off[b] * d;
-  for (int j = 0; j < I; j++)
-    for (int q = lane; q < d4; q += 32)
-      reinterpret_cast<float4*>(xin + (size_t)j * DP)[q] = reinterpret_cast<const float4*>(gin + (size_t)j * d)[q];
-  {
-    float4 v[kOMax][DCH];
-#pragma unroll
-    for (int i = 0; i < kOMax; i++)
-#pragma unroll
-      for (int t = 0; t < DCH; t++) {
-        const int q = lane + 32 * t;
-        v[i][t] = (i < O && q < d4) ? reinterpret_cast<const float4*>(gout + (size_t)i * d)[q]
-                                    : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-    store_out_interleaved<kOMax, DCH>(v, O, d, outI);
-  }
-  for (int i = lane; i < O; i += 32) meta[i] = out_meta_all[out_off[b] + i];
-  __syncwarp();
-  auto in_ptr = [&](int j) -> const float* { return xin + (size_t)j * DP; };
-  float loss = 0.f;
-  forward_gradient<kOMax>(I, first, O, d, in_ptr, outI, meta, exp_s, alpha[b], corrP, false, loss);
-  float4 md[kOMax][DCH];
-  if (!kRound) {
-    float* gdin = d_in + in_off[b] * d;
-    backward<kOMax, DCH>(I, O, d, in_ptr, [&](int pp, int q, float4& r0, float4& r1) { out_chunk_pair(outI, d, pp, q, r0, r1); }, corrP, md,
-                         [&](int j, int q, float4 a) { reinterpret_cast<float4*>(gdin + (size_t)j * d)[q] = a; });
-    float* gdout = d_out + out_off[b] * d;
-#pragma unroll
-    for (int i = 0; i < kOMax; i++)
-#pragma unroll
-      for (int t = 0; t < DCH; t++) {
-        const int q = lane + 32 * t;
-        if (i < O && q < d4) reinterpret_cast<float4*>(gdout + (size_t)i * d)[q] = md[i][t];
-      }
+  int64_t i_at, o_at;
+  if (in_off) {
+    i_at = in_off[b], o_at = out_off[b];
   } else {
-    // rows j of the inputs: event key EV_WALK0 of minibatch b; row index = j (outputs: the
-    // key EV_NEG, row index = i) -- the same rounding rule and hash as the trainers' stores
-    const uint64_t ev_in = sr_event_key(sr_seed, EV_WALK0, 0u, (uint64_t)b);
-    const uint64_t ev_out = sr_event_key(sr_seed, EV_NEG, 0u, (uint64_t)b);
-    uint16_t* gin16 = reinterpret_cast<uint16_t*>(d_in) + in_off[b] * d;
-    backward<kOMax, DCH>(I, O, d, in_ptr, [&](int pp, int q, float4& r0, float4& r1) { out_chunk_pair(outI, d, pp, q, r0, r1); }, corrP, md,
-                         [&](int j, int q, float4 a) {
-                           const float4 x = reinterpret_cast<const float4*>(gin + (size_t)j * d)[q];
-                           RowIO<STORE_BF16>::store4(gin16, j, d, q, add4(x, a), ev_in);
-                         });
-    uint16_t* gout16 = reinterpret_cast<uint16_t*>(d_out) + out_off[b] * d;
+    i_at = o_at = 0;  // (a negative count adds nothing, as in prefix_offsets_kernel)
+    for (int k = threadIdx.x; k < b; k += kMbThreads) {
+      i_at += max(in_count[k], 0);
+      o_at += max(out_count[k], 0);
+    }
+    block_sum2(i_at, o_at, sums);
+  }
+  const int DP = d + 4, d4 = d >> 2;  // rows 4 banks apart
+  constexpr int CS = kOMax;
+  float* xin = smem;
+  float* out = xin + (size_t)imax * DP;
+  float* corr = out + (size_t)kOMax * DP;
+  const float* gin = in_rows + i_at * d;
+  const float* gout = out_rows + o_at * d;
+  for (int e = threadIdx.x; e < (I + O) * d4; e += kMbThreads) {
+    const int r = e / d4, q = e - r * d4;
+    const float4 v = r < I ? reinterpret_cast<const float4*>(gin)[e] : reinterpret_cast<const float4*>(gout)[e - I * d4];
+    reinterpret_cast<float4*>(r < I ? xin + r * DP : out + (r - I) * DP)[q] = v;
+  }
+  __syncthreads();
+  // dot products of outputs 2p, 2p + 1 with input j, then their gradients (dsgl.hpp:1243-1272)
+  const float al = alpha[b];
+  const int cols = (I + 31) & ~31;  // a warp's lanes hold different inputs against the same outputs
+  for (int t = threadIdx.x; t < cols * ((O + 1) >> 1); t += kMbThreads) {
+    const int p = t / cols, j = t - p * cols;
+    if (j >= I) continue;
+    const float4* x = reinterpret_cast<const float4*>(xin + j * DP);
+    const float4* oa = reinterpret_cast<const float4*>(out + 2 * p * DP);
+    const float4* ob = reinterpret_cast<const float4*>(out + (2 * p + 1 < O ? 2 * p + 1 : 2 * p) * DP);
+    float f[2] = {0.f, 0.f};
+#pragma unroll 4
+    for (int k = 0; k < d4; k++) {
+      const float4 xv = x[k], u = oa[k], v = ob[k];
+      f[0] = __fmaf_rn(u.x, xv.x, f[0]);
+      f[1] = __fmaf_rn(v.x, xv.x, f[1]);
+      f[0] = __fmaf_rn(u.y, xv.y, f[0]);
+      f[1] = __fmaf_rn(v.y, xv.y, f[1]);
+      f[0] = __fmaf_rn(u.z, xv.z, f[0]);
+      f[1] = __fmaf_rn(v.z, xv.z, f[1]);
+      f[0] = __fmaf_rn(u.w, xv.w, f[0]);
+      f[1] = __fmaf_rn(v.w, xv.w, f[1]);
+    }
 #pragma unroll
-    for (int i = 0; i < kOMax; i++)
-#pragma unroll
-      for (int t = 0; t < DCH; t++) {
-        const int q = lane + 32 * t;
-        if (i < O && q < d4) {
-          const float4 o = reinterpret_cast<const float4*>(gout + (size_t)i * d)[q];
-          RowIO<STORE_BF16>::store4(gout16, i, d, q, add4(o, md[i][t]), ev_out);
-        }
-      }
+    for (int h = 0; h < 2; h++) {
+      const int i = 2 * p + h;
+      if (i < O)
+        corr[j * CS + i] = step_gradient(f[h], j < first ? (i == 0) : (i == O - 1), exp_table, al, out_meta_all[o_at + i]);
+    }
+  }
+  __syncthreads();
+  // event keys of the rounded rows: EV_WALK0 (inputs) and EV_NEG (outputs) of minibatch b, row
+  // index within the minibatch -- the trainers' rounding rule and hash
+  const uint64_t ev_in = kRound ? sr_event_key(sr_seed, EV_WALK0, 0u, (uint64_t)b) : 0;
+  const uint64_t ev_out = kRound ? sr_event_key(sr_seed, EV_NEG, 0u, (uint64_t)b) : 0;
+  uint16_t* gin16 = reinterpret_cast<uint16_t*>(d_in) + i_at * d;
+  uint16_t* gout16 = reinterpret_cast<uint16_t*>(d_out) + o_at * d;
+  for (int q = lane; q < d4; q += 32) {
+    // outputMd_i = sum_j g_ij x_j, in input order
+    for (int i = warp; i < O; i += kMbThreads / 32) {
+      float4 m = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+      for (int j = 0; j < I; j++) m = fma4s(corr[j * CS + i], reinterpret_cast<const float4*>(xin + j * DP)[q], m);
+      if (kRound)
+        RowIO<STORE_BF16>::store4(gout16, i, d, q, add4(reinterpret_cast<const float4*>(out + i * DP)[q], m), ev_out);
+      else
+        reinterpret_cast<float4*>(d_out + (o_at + i) * d)[q] = m;
+    }
+    // input j's update = sum_i g_ij o_i, in output order
+    for (int j = warp; j < I; j += kMbThreads / 32) {
+      float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+      for (int i = 0; i < O; i++) a = fma4s(corr[j * CS + i], reinterpret_cast<const float4*>(out + i * DP)[q], a);
+      if (kRound)
+        RowIO<STORE_BF16>::store4(gin16, j, d, q, add4(reinterpret_cast<const float4*>(xin + j * DP)[q], a), ev_in);
+      else
+        reinterpret_cast<float4*>(d_in + (i_at + j) * d)[q] = a;
+    }
   }
 }
 
@@ -163,18 +212,47 @@ __global__ void max_walk_kernel(const int32_t* rows, int64_t n, int32_t* out) {
   if ((threadIdx.x & 31) == 0 && best > 0) atomicMax(out, best);
 }
 
-// A negative count (rejected by its own minibatch) adds nothing, so no later minibatch's
-// offset points before the start of the caller's row arrays.
-__global__ void prefix_offsets_kernel(const int32_t* cnt_a, const int32_t* cnt_b, int n, int64_t* off_a,
-                                      int64_t* off_b) {
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    int64_t a = 0, bb = 0;
-    for (int i = 0; i < n; i++) {
-      off_a[i] = a;
-      off_b[i] = bb;
-      a += cnt_a[i] > 0 ? cnt_a[i] : 0;
-      bb += cnt_b[i] > 0 ? cnt_b[i] : 0;
+// Exclusive prefixes of two count arrays, one block: each thread sums its run of consecutive
+// counts, the runs are scanned, the runs are written.  A negative count (rejected by its own
+// minibatch) adds nothing, so no later minibatch's offset points before the start of the
+// caller's row arrays.
+constexpr int kPrefixThreads = 1024;
+__global__ void __launch_bounds__(kPrefixThreads) prefix_offsets_kernel(const int32_t* cnt_a, const int32_t* cnt_b, int n,
+                                                                        int64_t* off_a, int64_t* off_b) {
+  __shared__ int64_t wa[32], wb[32];
+  const int lane = lane_id(), warp = threadIdx.x >> 5;
+  const int run = (n + kPrefixThreads - 1) / kPrefixThreads;
+  const int lo = min((int64_t)threadIdx.x * run, (int64_t)n), hi = min((int64_t)lo + run, (int64_t)n);
+  int64_t a = 0, b = 0;
+  for (int i = lo; i < hi; i++) {
+    a += max(cnt_a[i], 0);
+    b += max(cnt_b[i], 0);
+  }
+  int64_t ia = a, ib = b;  // inclusive over the warp, then the block
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int64_t u = __shfl_up_sync(kFull, ia, o), v = __shfl_up_sync(kFull, ib, o);
+    if (lane >= o) ia += u, ib += v;
+  }
+  if (lane == 31) wa[warp] = ia, wb[warp] = ib;
+  __syncthreads();
+  if (warp == 0) {
+    int64_t u = wa[lane], v = wb[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int64_t x = __shfl_up_sync(kFull, u, o), y = __shfl_up_sync(kFull, v, o);
+      if (lane >= o) u += x, v += y;
     }
+    wa[lane] = u, wb[lane] = v;
+  }
+  __syncthreads();
+  a = ia - a + (warp ? wa[warp - 1] : 0);
+  b = ib - b + (warp ? wb[warp - 1] : 0);
+  for (int i = lo; i < hi; i++) {
+    off_a[i] = a;
+    off_b[i] = b;
+    a += max(cnt_a[i], 0);
+    b += max(cnt_b[i], 0);
   }
 }
 
@@ -273,35 +351,35 @@ cudaError_t launch_max_walk(const int32_t* rows, int64_t n, int32_t* out, cudaSt
   return cudaGetLastError();
 }
 
+namespace {
+template <bool kRound>
+cudaError_t minibatch_launch(int d, int n, int imax, const int32_t* in_count, const int32_t* in_first,
+                             const int32_t* out_count, const int32_t* out_meta, const float* alpha,
+                             const float* in_rows, const float* out_rows, float* d_in, float* d_out, uint64_t sr_seed,
+                             const float* exp_table, int64_t* offsets, int32_t* status, cudaStream_t s) {
+  if (n == 0) return cudaSuccess;
+  // small calls: a launch saved is worth the counts being read by every block
+  int64_t* in_off = n <= kMbOwnPrefix ? nullptr : offsets;
+  int64_t* out_off = n <= kMbOwnPrefix ? nullptr : offsets + n;
+  if (in_off) prefix_offsets_kernel<<<1, kPrefixThreads, 0, s>>>(in_count, out_count, n, in_off, out_off);
+  const size_t smem = sizeof(float) * ((size_t)(imax + kOMax) * (d + 4) + (size_t)imax * kOMax);
+  cudaError_t e = cudaFuncSetAttribute(minibatch_kernel<kRound>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  minibatch_kernel<kRound><<<n, kMbThreads, smem, s>>>(d, imax, kOMax, in_count, in_first, out_count, out_meta, alpha,
+                                                       in_off, out_off, in_rows, out_rows, d_in, d_out, exp_table,
+                                                       status, sr_seed);
+  return cudaGetLastError();
+}
+}  // namespace
+
 cudaError_t launch_minibatch_bf16(int d, int n, int imax, const int32_t* in_count, const int32_t* in_first,
                                   const int32_t* out_count, const int32_t* out_meta, const float* alpha,
                                   const float* in_rows, const float* out_rows, uint16_t* new_in, uint16_t* new_out,
                                   uint64_t sr_seed, const float* exp_table, int64_t* offsets, int32_t* status,
                                   cudaStream_t s) {
-  if (n == 0) return cudaSuccess;
-  int64_t* in_off = offsets;
-  int64_t* out_off = offsets + n;
-  prefix_offsets_kernel<<<1, 1, 0, s>>>(in_count, out_count, n, in_off, out_off);
-  const int DP = d + 4;
-  const size_t smem = sizeof(float) * (1004 + (size_t)imax * DP + (size_t)kOMax * d +
-                                       (size_t)imax * (kOMax + 2) * 2 + kOMax + 4);
-  float* a = reinterpret_cast<float*>(new_in);
-  float* b = reinterpret_cast<float*>(new_out);
-  cudaError_t e;
-  if (d > 128) {
-    e = cudaFuncSetAttribute(minibatch_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    minibatch_kernel<2, true><<<n, 32, smem, s>>>(d, imax, kOMax, in_count, in_first, out_count, out_meta, alpha,
-                                                  in_off, out_off, in_rows, out_rows, a, b, exp_table, status,
-                                                  sr_seed);
-  } else {
-    e = cudaFuncSetAttribute(minibatch_kernel<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    minibatch_kernel<1, true><<<n, 32, smem, s>>>(d, imax, kOMax, in_count, in_first, out_count, out_meta, alpha,
-                                                  in_off, out_off, in_rows, out_rows, a, b, exp_table, status,
-                                                  sr_seed);
-  }
-  return cudaGetLastError();
+  return minibatch_launch<true>(d, n, imax, in_count, in_first, out_count, out_meta, alpha, in_rows, out_rows,
+                                reinterpret_cast<float*>(new_in), reinterpret_cast<float*>(new_out), sr_seed, exp_table,
+                                offsets, status, s);
 }
 
 cudaError_t launch_minibatch(int d, int n, int imax, int omax, const int32_t* in_count,
@@ -309,27 +387,9 @@ cudaError_t launch_minibatch(int d, int n, int imax, int omax, const int32_t* in
                              const float* alpha, const float* in_rows, const float* out_rows, float* d_in,
                              float* d_out, const float* exp_table, int64_t* offsets, int32_t* status,
                              cudaStream_t s) {
-  if (n == 0) return cudaSuccess;
-  int64_t* in_off = offsets;
-  int64_t* out_off = offsets + n;
-  prefix_offsets_kernel<<<1, 1, 0, s>>>(in_count, out_count, n, in_off, out_off);
-  const int DP = d + 4;
   (void)omax;
-  const size_t smem = sizeof(float) * (1004 + (size_t)imax * DP + (size_t)kOMax * d +
-                                       (size_t)imax * (kOMax + 2) * 2 + kOMax + 4);
-  cudaError_t e;
-  if (d > 128) {
-    e = cudaFuncSetAttribute(minibatch_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    minibatch_kernel<2><<<n, 32, smem, s>>>(d, imax, omax, in_count, in_first, out_count, out_meta, alpha,
-                                            in_off, out_off, in_rows, out_rows, d_in, d_out, exp_table, status);
-  } else {
-    e = cudaFuncSetAttribute(minibatch_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    minibatch_kernel<1><<<n, 32, smem, s>>>(d, imax, omax, in_count, in_first, out_count, out_meta, alpha,
-                                            in_off, out_off, in_rows, out_rows, d_in, d_out, exp_table, status);
-  }
-  return cudaGetLastError();
+  return minibatch_launch<false>(d, n, imax, in_count, in_first, out_count, out_meta, alpha, in_rows, out_rows, d_in,
+                                 d_out, 0, exp_table, offsets, status, s);
 }
 
 }  // namespace sgns

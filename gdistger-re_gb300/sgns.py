@@ -367,10 +367,14 @@ def edge_common_neighbors(indptr, indices, cn, stream=0):
                                             cn.data_ptr() if E else None, ctypes.c_void_p(stream)))
 
 
+# Bytes that info_walks takes for a moment to make a corpus of unknown size in one call.
+_WALK_ROOM = 4 << 30
+
+
 def info_walks(indptr, indices, cn, walker_num, min_length=20, max_length=80, r_threshold=0.999, seed=1,
                corpus=None, stream=0, trace=1):
     """sgns_info_walks on device tensors.  corpus: int32 device tensor to fill (None: a new
-    one of the exact size, after a counting call).  Returns (corpus, n_tokens)."""
+    one of the exact size).  Returns (corpus, n_tokens)."""
     import torch
 
     V, E = int(indptr.numel()) - 1, int(indices.numel())
@@ -378,7 +382,17 @@ def info_walks(indptr, indices, cn, walker_num, min_length=20, max_length=80, r_
                     r_threshold=float(r_threshold), seed=int(seed), trace_steps=int(trace))
     n = ctypes.c_int64()
     args = (indptr.data_ptr(), indices.data_ptr() if E else None, cn.data_ptr() if E else None, V, E)
-    if corpus is None:
+    most = o.walker_num * (o.max_length + 1)
+    if corpus is None and 0 < 4 * most <= _WALK_ROOM:  # one call into room for the longest walks
+        try:
+            room = torch.empty(most, dtype=torch.int32, device=indptr.device)
+        except torch.cuda.OutOfMemoryError:
+            room = None
+        if room is not None:
+            _check(lib().sgns_info_walks(ctypes.byref(o), *args, room.data_ptr(), most, ctypes.byref(n),
+                                         ctypes.c_void_p(stream)))
+            return room[:n.value].clone(), n.value
+    if corpus is None:  # a counting call first: the length pass runs twice
         _check(lib().sgns_info_walks(ctypes.byref(o), *args, None, 0, ctypes.byref(n), ctypes.c_void_p(stream)))
         corpus = torch.empty(max(n.value, 1), dtype=torch.int32, device=indptr.device)
     _check(lib().sgns_info_walks(ctypes.byref(o), *args, corpus.data_ptr(), int(corpus.numel()), ctypes.byref(n),
