@@ -10,9 +10,12 @@
 // checked against finite differences).
 //
 // Sparse output: every row referenced by the batch appears once, in ascending row order.
-// Rows are marked in a V-sized array, the marks are prefix-summed (row -> compact slot),
-// the compact gradient rows are zeroed, and each minibatch adds its row gradients into
-// its rows' slots.
+// References are marked in bitmaps, 32 rows to a 16-byte word (RowMark): whether a row is
+// referenced, whether more than once, and -- after a scan of the words -- how many referenced
+// rows come before it.  A row's compact slot is then one word read from L2 (2 MB for 4M rows,
+// where a slot per row took 16 MB and four passes over it).  Rows referenced more than once are
+// zeroed and take their gradients by atomic adds; the others are stored once, which saves the
+// zeroing, the atomic and the read behind it.
 //
 // Gradient kernels.  adjoint_pipe_kernel (tables whose rows are whole 16-byte chunks at
 // 16-byte aligned addresses) runs persistent warps that copy the next minibatch's rows
@@ -27,7 +30,7 @@
 //   * the gradient rows are column-parallel (lane l owns columns 4l..4l+3 of each
 //     128-column chunk) and leave with one 16-byte atomic add per lane (red.global.add of
 //     four floats; fp64 adds element by element);
-//   * the loss is reduced per warp, then per block, with one fp64 atomic per block;
+//   * the loss is reduced per warp into 256 fp64 sums;
 //   * sizes and ids are checked on the device (status bits), so a call makes no host round
 //     trip before its launches.
 #include <cuda_runtime.h>
@@ -93,19 +96,49 @@ __device__ __forceinline__ void pair_terms(double f, int label, double meta, dou
 __device__ __forceinline__ float fma_t(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double fma_t(double a, double b, double c) { return __fma_rn(a, b, c); }
 
-__device__ __forceinline__ void atomic_add4(float* dst, const float (&v)[4]) {
-  atomicAdd(reinterpret_cast<float4*>(dst), make_float4(v[0], v[1], v[2], v[3]));
-}
 __device__ __forceinline__ void atomic_add4(double* dst, const double (&v)[4]) {
 #pragma unroll
   for (int k = 0; k < 4; k++) atomicAdd(dst + k, v[k]);
 }
 
+// 32 consecutive rows of a table
+struct __align__(16) RowMark {
+  uint32_t once;   // referenced
+  uint32_t more;   // referenced more than once
+  int32_t before;  // referenced rows before the word
+  int32_t pad;
+};
+// A referenced row's slot; the sign bit says that the batch references it once.
+constexpr int32_t kSole = (int32_t)0x80000000u;
+__device__ __forceinline__ int32_t row_slot(const RowMark* marks, int32_t row) {
+  const int4 w = __ldg(reinterpret_cast<const int4*>(marks) + (row >> 5));
+  const uint32_t bit = 1u << (row & 31);
+  return (w.z + __popc((uint32_t)w.x & (bit - 1))) | (((uint32_t)w.y & bit) ? 0 : kSole);
+}
+__device__ __forceinline__ void mark_row(RowMark* marks, int32_t row) {
+  RowMark* w = marks + (row >> 5);
+  const uint32_t bit = 1u << (row & 31);
+  if (__ldcg(&w->more) & bit) return;  // the many references of a popular row cost a read each
+  if (atomicOr(&w->once, bit) & bit) atomicOr(&w->more, bit);
+}
+// The first kHotRows rows of each table (tables are sorted by frequency, and a few thousand
+// rows take half of a power law's references) are marked in the block's shared memory and
+// merged once per block: their marks lie in a few cache lines that every reference would meet in.
+constexpr int kHotRows = 16384, kHotWords = kHotRows / 32, kHotThreads = 512;
+
+// info words of a call (device memory): distinct input and output rows, status bits, largest
+// input and output count, blocks of the gradient kernel that are done
+enum { INFO_IN = 0, INFO_OUT, INFO_STATUS, INFO_IMAX, INFO_OMAX, INFO_DONE, INFO_WORDS = 8 };
+
 // Marks the rows of every minibatch (one warp per minibatch, one lane per id), checks its
-// extents and records the largest input and output counts (dims[0], dims[1]).
-__global__ void mark_rows_kernel(int n, const int32_t* in_ptr, const int32_t* in_ids, const int32_t* in_first,
-                                 const int32_t* out_ptr, const int32_t* out_ids, int64_t V, int32_t* mark_in,
-                                 int32_t* mark_out, int32_t* status, int32_t* dims) {
+// extents and records the largest input and output counts.
+__global__ void __launch_bounds__(kHotThreads) mark_rows_kernel(int n, const int32_t* in_ptr, const int32_t* in_ids,
+                                                                const int32_t* in_first, const int32_t* out_ptr,
+                                                                const int32_t* out_ids, int64_t V, RowMark* mark_in,
+                                                                RowMark* mark_out, int32_t* info) {
+  __shared__ uint32_t hot[2][2][kHotWords];  // table; referenced, more than once
+  for (int k = threadIdx.x; k < 4 * kHotWords; k += kHotThreads) (&hot[0][0][0])[k] = 0u;
+  __syncthreads();
   const int lane = lane_id();
   const int warps = (int)((gridDim.x * blockDim.x) >> 5);
   int imax = 0, omax = 0;
@@ -113,119 +146,158 @@ __global__ void mark_rows_kernel(int n, const int32_t* in_ptr, const int32_t* in
     const int i0 = in_ptr[b], i1 = in_ptr[b + 1], o0 = out_ptr[b], o1 = out_ptr[b + 1];
     if (i0 < 0 || o0 < 0 || i1 - i0 < 0 || i1 - i0 > kIMax || o1 - o0 < 0 || o1 - o0 > kOMax ||
         in_first[b] < 0 || in_first[b] > i1 - i0) {
-      if (lane == 0) atomicOr(status, kBadSize);
+      if (lane == 0) atomicOr(&info[INFO_STATUS], kBadSize);
       continue;
     }
     imax = max(imax, i1 - i0);
     omax = max(omax, o1 - o0);
-    for (int t = i0 + lane; t < i1; t += 32) {
-      const int32_t r = in_ids[t];
-      if (r < 0 || r >= V) atomicOr(status, kBadId);
-      else mark_in[r] = 1;
-    }
-    for (int t = o0 + lane; t < o1; t += 32) {
-      const int32_t r = out_ids[t];
-      if (r < 0 || r >= V) atomicOr(status, kBadId);
-      else mark_out[r] = 1;
+    for (int t = lane; t < i1 - i0 + o1 - o0; t += 32) {
+      const int table = t >= i1 - i0;
+      const int32_t r = table ? out_ids[o0 + t - (i1 - i0)] : in_ids[i0 + t];
+      if (r < 0 || r >= V) {
+        atomicOr(&info[INFO_STATUS], kBadId);
+      } else if (r < kHotRows) {
+        const uint32_t bit = 1u << (r & 31);
+        if (!(*static_cast<volatile uint32_t*>(&hot[table][1][r >> 5]) & bit) &&
+            (atomicOr(&hot[table][0][r >> 5], bit) & bit))
+          atomicOr(&hot[table][1][r >> 5], bit);
+      } else {
+        mark_row(table ? mark_out : mark_in, r);
+      }
     }
   }
   imax = __reduce_max_sync(kFull, imax);
   omax = __reduce_max_sync(kFull, omax);
   if ((threadIdx.x & 31) == 0) {
-    atomicMax(&dims[0], imax);
-    atomicMax(&dims[1], omax);
+    atomicMax(&info[INFO_IMAX], imax);
+    atomicMax(&info[INFO_OMAX], omax);
+  }
+  __syncthreads();
+  for (int k = threadIdx.x; k < 2 * kHotWords; k += kHotThreads) {
+    const int table = k / kHotWords, word = k % kHotWords;
+    const uint32_t once = hot[table][0][word];
+    if (!once) continue;
+    RowMark* w = (table ? mark_out : mark_in) + word;
+    const uint32_t more = (atomicOr(&w->once, once) & once) | hot[table][1][word];
+    if (more) atomicOr(&w->more, more);
   }
 }
 
-// ---- inclusive scan of int32 marks: tiles of 4096, then the tile sums in one block -----
-constexpr int kScanThreads = 1024;
-constexpr int kScanItems = 4;
-constexpr int kScanTile = kScanThreads * kScanItems;
+// ---- slots: referenced rows per tile of words, then each tile's words and ids -------------
+constexpr int kMarkThreads = 256, kMarkItems = 4;
+constexpr int kMarkTile = kMarkThreads * kMarkItems;  // words of a tile: 32,768 rows
 
-__device__ __forceinline__ int32_t block_exclusive_prefix(int32_t run, int32_t* warp_sums, int32_t* total) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int32_t x = run;
+__device__ __forceinline__ int32_t block_sum(int32_t v, int32_t* scratch) {
+  v = __reduce_add_sync(kFull, v);
+  __syncthreads();
+  if (lane_id() == 0) scratch[threadIdx.x >> 5] = v;
+  __syncthreads();
+  int32_t t = 0;
+#pragma unroll
+  for (int k = 0; k < kMarkThreads / 32; k++) t += scratch[k];
+  return t;
+}
+
+// blockIdx.y: 0 = input table, 1 = output table
+__global__ void __launch_bounds__(kMarkThreads) count_tiles_kernel(const RowMark* marks, int64_t words, int32_t* sums,
+                                                                   int tiles) {
+  __shared__ int32_t scratch[kMarkThreads / 32];
+  marks += blockIdx.y * words;
+  const int64_t base = (int64_t)blockIdx.x * kMarkTile + threadIdx.x;
+  int32_t c = 0;
+#pragma unroll
+  for (int k = 0; k < kMarkItems; k++) {
+    const int64_t i = base + k * kMarkThreads;
+    if (i < words) c += __popc(marks[i].once);
+  }
+  c = block_sum(c, scratch);
+  if (threadIdx.x == 0) sums[blockIdx.y * tiles + blockIdx.x] = c;
+}
+
+__global__ void __launch_bounds__(kMarkThreads) emit_rows_kernel(RowMark* marks, int64_t words, const int32_t* sums,
+                                                                 int tiles, int32_t* in_ids, int32_t* out_ids,
+                                                                 int32_t* info) {
+  __shared__ int32_t scratch[kMarkThreads / 32], warp_total[kMarkThreads / 32];
+  marks += blockIdx.y * words;
+  sums += blockIdx.y * tiles;
+  int32_t* ids = blockIdx.y ? out_ids : in_ids;
+  int32_t before = 0;
+  for (int t = threadIdx.x; t < (int)blockIdx.x; t += kMarkThreads) before += sums[t];
+  before = block_sum(before, scratch);
+  // a thread's words are consecutive, so its ids are
+  const int64_t base = (int64_t)blockIdx.x * kMarkTile + (int64_t)threadIdx.x * kMarkItems;
+  uint32_t w[kMarkItems];
+  int32_t c = 0;
+#pragma unroll
+  for (int k = 0; k < kMarkItems; k++) {
+    w[k] = base + k < words ? marks[base + k].once : 0u;
+    c += __popc(w[k]);
+  }
+  const int lane = lane_id(), warp = threadIdx.x >> 5;
+  int32_t inc = c;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const int32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
-    if (lane >= o) x += y;
+    const int32_t t = __shfl_up_sync(kFull, inc, o);
+    if (lane >= o) inc += t;
   }
-  if (lane == 31) warp_sums[warp] = x;
+  if (lane == 31) warp_total[warp] = inc;
   __syncthreads();
-  if (warp == 0) {
-    int32_t s = lane < (int)(blockDim.x >> 5) ? warp_sums[lane] : 0;
+  for (int k = 0; k < warp; k++) before += warp_total[k];
+  int32_t at = before + inc - c;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int32_t y = __shfl_up_sync(0xFFFFFFFFu, s, o);
-      if (lane >= o) s += y;
+  for (int k = 0; k < kMarkItems; k++) {
+    if (base + k < words) {
+      marks[base + k].before = at;
+      for (uint32_t m = w[k]; m; m &= m - 1) ids[at++] = (int32_t)(32 * (base + k) + __ffs(m) - 1);
     }
-    warp_sums[lane] = s;
   }
-  __syncthreads();
-  *total = warp_sums[31];
-  return (x - run) + (warp > 0 ? warp_sums[warp - 1] : 0);
+  if (blockIdx.x == (unsigned)tiles - 1 && threadIdx.x == kMarkThreads - 1) info[blockIdx.y ? INFO_OUT : INFO_IN] = at;
 }
 
-__global__ void __launch_bounds__(kScanThreads) scan_tiles_kernel(int32_t* a, int64_t n, int32_t* tile_sums) {
-  __shared__ int32_t warp_sums[32];
-  const int64_t base = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems;
-  int32_t v[kScanItems];
-  int32_t run = 0;
-#pragma unroll
-  for (int k = 0; k < kScanItems; k++) {
-    v[k] = base + k < n ? a[base + k] : 0;
-    run += v[k];
-    v[k] = run;
-  }
-  int32_t total;
-  const int32_t prefix = block_exclusive_prefix(run, warp_sums, &total);
-#pragma unroll
-  for (int k = 0; k < kScanItems; k++)
-    if (base + k < n) a[base + k] = v[k] + prefix;
-  if (threadIdx.x == 0) tile_sums[blockIdx.x] = total;
-}
-
-// one block: tile sums -> exclusive tile prefixes, in rounds of kScanThreads
-__global__ void __launch_bounds__(kScanThreads) scan_tile_sums_kernel(int32_t* tile_sums, int64_t ntiles) {
-  __shared__ int32_t warp_sums[32];
-  __shared__ int32_t carry;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  for (int64_t base = 0; base < ntiles; base += kScanThreads) {
-    const int64_t i = base + threadIdx.x;
-    const int32_t v = i < ntiles ? tile_sums[i] : 0;
-    int32_t total;
-    const int32_t ex = block_exclusive_prefix(v, warp_sums, &total);
-    const int32_t c0 = carry;
-    if (i < ntiles) tile_sums[i] = c0 + ex;
-    __syncthreads();
-    if (threadIdx.x == 0) carry = c0 + total;
-    __syncthreads();
-  }
-}
-
-// adds the tile prefixes; marked rows (incl[r] - incl[r-1] == 1) -> ids[incl[r] - 1] = r
-// (the previous row's value is recomputed from its own tile prefix, so one pass suffices)
-__global__ void add_prefix_emit_kernel(const int32_t* a, int64_t n, const int32_t* tile_prefix, int32_t* ids) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int32_t v = a[i] + tile_prefix[i / kScanTile];
-    const int32_t prev = i == 0 ? 0 : a[i - 1] + tile_prefix[(i - 1) / kScanTile];
-    if (v != prev) ids[v - 1] = (int32_t)i;
-  }
-}
-
-// final pass: a[i] += its tile prefix (after the ids were emitted from the tile-local values)
-__global__ void add_prefix_kernel(int32_t* a, int64_t n, const int32_t* tile_prefix) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    a[i] += tile_prefix[i / kScanTile];
-}
-
-// zeroes the first incl[V-1] rows of a gradient array (the rows the call emits)
+// zeroes the gradient rows that take atomic adds: one warp per word of marks
 template <class T>
-__global__ void zero_rows_kernel(T* g, const int32_t* incl_last, int d) {
-  const int64_t n = (int64_t)(*incl_last) * d;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    g[i] = T(0);
+__global__ void __launch_bounds__(256) zero_rows_kernel(const RowMark* marks, int64_t words, T* g_in, T* g_out, int d) {
+  const int lane = lane_id();
+  const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < 2 * words; i += warps) {
+    const int4 w = __ldg(reinterpret_cast<const int4*>(marks) + i);
+    T* g = i < words ? g_in : g_out;
+    for (uint32_t m = (uint32_t)w.y; m; m &= m - 1) {
+      const uint32_t below = (m & (0u - m)) - 1;
+      T* row = g + (int64_t)(w.z + __popc((uint32_t)w.x & below)) * d;
+      if (sizeof(T) == 4 && (d & 3) == 0) {
+        for (int c = lane; c < (d >> 2); c += 32) reinterpret_cast<float4*>(row)[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+      } else {
+        for (int c = lane; c < d; c += 32) row[c] = T(0);
+      }
+    }
+  }
+}
+
+__device__ __forceinline__ void add_row4(float* g, int32_t slot, int d, int q, const float (&v)[4]) {
+  // a store or a vector add by predicate: a branch per row cost more than it saved
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.lt.s32 p, %0, 0;\n\t"
+      "@p st.global.v4.f32 [%1], {%2, %3, %4, %5};\n\t"
+      "@!p red.relaxed.gpu.global.add.v4.f32 [%1], {%2, %3, %4, %5};\n\t}"
+      ::"r"(slot), "l"(g + (size_t)(slot & ~kSole) * d + 4 * q), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3])
+      : "memory");
+}
+__device__ __forceinline__ void add_row4(double* g, int32_t slot, int d, int q, const double (&v)[4]) {
+  double* dst = g + (size_t)(slot & ~kSole) * d + 4 * q;
+  if (slot < 0) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) dst[k] = v[k];
+  } else {
+    atomic_add4(dst, v);
+  }
+}
+template <class T>
+__device__ __forceinline__ void add_row1(T* g, int32_t slot, int d, int q, T v) {
+  T* dst = g + (size_t)(slot & ~kSole) * d + q;
+  if (slot < 0) *dst = v;
+  else atomicAdd(dst, v);
 }
 
 // Shared memory of one warp: input rows (imax x DP), output rows (omax x d), coefficients
@@ -259,7 +331,7 @@ template <int DT, int VW, int OMX>
 __global__ void __launch_bounds__(32 * kWarpsPerBlock) adjoint_kernel(
     int d, int n, int imax, int omax, const int32_t* in_ptr, const int32_t* in_ids, const int32_t* in_first,
     const int32_t* out_ptr, const int32_t* out_ids, const int32_t* out_meta, const void* wih, const void* woh,
-    int64_t V, const int32_t* incl_in, const int32_t* incl_out, typename Elem<DT>::T* g_in,
+    int64_t V, const RowMark* mark_in, const RowMark* mark_out, typename Elem<DT>::T* g_in,
     typename Elem<DT>::T* g_out, double* loss_parts) {
   typedef typename Elem<DT>::T T;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -281,7 +353,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) adjoint_kernel(
       const int32_t r = j < I ? in_ids[i0 + j] : out_ids[o0 + j - I];
       ok &= r >= 0 && r < V;
       // the row's gradient slot, looked up now so the atomics below wait on nothing
-      if (r >= 0 && r < V) slot[j] = (j < I ? incl_in[r] : incl_out[r]) - 1;
+      if (r >= 0 && r < V) slot[j] = row_slot(j < I ? mark_in : mark_out, r);
     }
   }
   if (!__all_sync(kFull, ok)) return;
@@ -359,7 +431,6 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) adjoint_kernel(
   __syncwarp();
   // dL/dWih[x_j] = sum_i coef_ij Woh[o_i], column-parallel
   for (int j = 0; j < I; j++) {
-    T* dst = g_in + (size_t)slot[j] * d;
     for (int q = lane; q < nq; q += 32) {
       T acc[4] = {0, 0, 0, 0};
       for (int i = 0; i < O; i++) {
@@ -370,13 +441,12 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) adjoint_kernel(
 #pragma unroll
         for (int t = 0; t < VW; t++) acc[t] = fma_t(c, ov[t], acc[t]);
       }
-      if (VW == 4) atomic_add4(dst + 4 * q, acc);
-      else atomicAdd(dst + q, acc[0]);
+      if (VW == 4) add_row4(g_in, slot[j], d, q, acc);
+      else add_row1(g_in, slot[j], d, q, acc[0]);
     }
   }
   // dL/dWoh[o_i] = sum_j coef_ij Wih[x_j]
   for (int i = 0; i < O; i++) {
-    T* dst = g_out + (size_t)slot[I + i] * d;
     for (int q = lane; q < nq; q += 32) {
       T acc[4] = {0, 0, 0, 0};
       for (int j = 0; j < I; j++) {
@@ -387,8 +457,8 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) adjoint_kernel(
 #pragma unroll
         for (int t = 0; t < VW; t++) acc[t] = fma_t(c, xv[t], acc[t]);
       }
-      if (VW == 4) atomic_add4(dst + 4 * q, acc);
-      else atomicAdd(dst + q, acc[0]);
+      if (VW == 4) add_row4(g_out, slot[I + i], d, q, acc);
+      else add_row1(g_out, slot[I + i], d, q, acc[0]);
     }
   }
   for (int sh = 16; sh > 0; sh >>= 1) loss += __shfl_xor_sync(kFull, loss, sh);
@@ -402,8 +472,12 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) adjoint_kernel(
 // L2 only) behind the current ones or at the ring's start when they fit beside them, so
 // their gathers overlap the backward; otherwise they are copied once the backward is
 // done.  A ring of one minibatch leaves room for more resident warps, which measured
-// faster than a second full buffer (12 warps per SM against 7 at d = 128, bf16, K = 5:
-// 2.08 against 2.86 ms per call on the 4M-vertex case).  The next minibatch's ids are
+// faster than a second full buffer (16 warps per SM against 7 at d = 128, bf16, K = 5).
+// Measured on the 4M-vertex case (200,000 minibatches, d = 128, bf16): 1,052 us with 12 warps,
+// the output rows widened into shared memory and every gradient an atomic; 845 us with 16
+// warps, the rows read from the ring and sole references stored.  Of a call's 1,048 us (1,550
+// before) the marks take 82, the slots and ids 29, the zeroed rows 46.  What bounds the kernel:
+// issue (57% of cycles, 2,670 warp instructions per minibatch), then its dependent chains.  The next minibatch's ids are
 // loaded at the top of an iteration, its gradient slots with its copies, and the extents
 // one minibatch further ahead.  Rows stay in their storage format in the ring (row stride
 // = row bytes + 16, so lanes reading different rows at one column hit different banks);
@@ -458,11 +532,13 @@ __host__ __device__ inline PipeLayout pipe_layout(int dtype, int d, int imax, in
   L.CS = (omx + 3) & ~3;
   L.buf = ring * L.RS;
   L.ofp = L.buf;
-  L.coef = L.ofp + omx * d * tb;
+  L.coef = L.ofp + (dtype == 1 ? 0 : omx * d * tb);  // bf16 rows are read from the ring
   L.slot = L.coef + imax * L.CS * tb;
   L.bytes = (L.slot + 4 * (imax + omax) + 15) & ~15;
   return L;
 }
+
+constexpr int kPipeSmem = 232448 - 64;  // a block's shared memory less the kernel's own few bytes
 
 // minibatch extents: i0, I, o0, O, first
 struct Extent {
@@ -574,12 +650,11 @@ __device__ __forceinline__ void forward_mma_bf16(const unsigned char* buf, int R
 }
 
 template <int DT, int OMX>
-__global__ void __launch_bounds__(256) adjoint_pipe_kernel(
+__global__ void __launch_bounds__(256, DT == 2 || OMX > 7 ? 1 : 2) adjoint_pipe_kernel(
     int d, int n, int imax, int omax, int ring, const int32_t* in_ptr, const int32_t* in_ids,
     const int32_t* in_first, const int32_t* out_ptr, const int32_t* out_ids, const int32_t* out_meta,
-    const void* wih, const void* woh, int64_t V, const int32_t* incl_in, const int32_t* incl_out,
-    typename Pipe<DT>::T* g_in,
-    typename Pipe<DT>::T* g_out, double* loss_parts) {
+    const void* wih, const void* woh, int64_t V, const RowMark* mark_in, const RowMark* mark_out,
+    typename Pipe<DT>::T* g_in, typename Pipe<DT>::T* g_out, double* loss_parts, int32_t* info, double* loss_out) {
   typedef typename Pipe<DT>::T T;
   constexpr int EB = Pipe<DT>::kBytes;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -630,7 +705,7 @@ __global__ void __launch_bounds__(256) adjoint_pipe_kernel(
 #pragma unroll
     for (int m = 0; m < 3; m++) {
       const int j = lane + 32 * m;
-      sl[m] = j < e.I ? incl_in[id[m]] - 1 : j < e.I + e.O ? incl_out[id[m]] - 1 : 0;
+      sl[m] = j < e.I + e.O ? row_slot(j < e.I ? mark_in : mark_out, id[m]) : 0;
     }
   };
 
@@ -665,15 +740,17 @@ __global__ void __launch_bounds__(256) adjoint_pipe_kernel(
     __syncwarp();
     const int I = cur.I, O = cur.O;
     if (cur_ok) {
-      // widen the output rows once (column-parallel); rows O .. OMX-1 are zero, so the
-      // products below run over the kernel's full output capacity without tests
-      for (int i = 0; i < OMX; i++)
-        for (int q = lane; q < nq; q += 32) {
-          T v[4] = {0, 0, 0, 0};
-          if (i < O) Pipe<DT>::chunk4(buf + (size_t)(I + i) * L.RS + 4 * q * EB, v);
-          sts4(ofp + (size_t)i * d + 4 * q, v);
-        }
-      __syncwarp();
+      if constexpr (DT != 1) {
+        // copy the output rows once (column-parallel); rows O .. OMX-1 are zero, so the
+        // products below run over the kernel's full output capacity without tests
+        for (int i = 0; i < OMX; i++)
+          for (int q = lane; q < nq; q += 32) {
+            T v[4] = {0, 0, 0, 0};
+            if (i < O) Pipe<DT>::chunk4(buf + (size_t)(I + i) * L.RS + 4 * q * EB, v);
+            sts4(ofp + (size_t)i * d + 4 * q, v);
+          }
+        __syncwarp();
+      }
       if constexpr (DT == 1) {
         forward_mma_bf16<OMX>(buf, L.RS, d, I, O, cur.first, out_meta + cur.o0, coef, L.CS, loss);
       } else {
@@ -773,18 +850,23 @@ __global__ void __launch_bounds__(256) adjoint_pipe_kernel(
                 ao[i][t] = fma_t(c, xv[t], ao[i][t]);
               }
             }
-            atomic_add4(g_in + (size_t)slot[j] * d + 4 * q, ai);
+            add_row4(g_in, slot[j], d, q, ai);
           }
 #pragma unroll
           for (int i = 0; i < OMX; i++)
-            if (i < O) atomic_add4(g_out + (size_t)slot[I + i] * d + 4 * q, ao[i]);
+            if (i < O) add_row4(g_out, slot[I + i], d, q, ao[i]);
         } else {
           // packed fp32 pairs: the same fused multiply-adds in the same order
           float2 ov[OMX][2], ao[OMX][2];
 #pragma unroll
           for (int i = 0; i < OMX; i++) {
-            const float4 o4 = *reinterpret_cast<const float4*>(ofp + (size_t)i * d + 4 * q);
-            ov[i][0] = make_float2(o4.x, o4.y), ov[i][1] = make_float2(o4.z, o4.w);
+            float o4[4] = {0.f, 0.f, 0.f, 0.f};
+            if constexpr (DT == 1) {
+              if (i < O) Pipe<DT>::chunk4(buf + (size_t)(I + i) * L.RS + 4 * q * EB, o4);
+            } else {
+              lds4(ofp + (size_t)i * d + 4 * q, o4);
+            }
+            ov[i][0] = make_float2(o4[0], o4[1]), ov[i][1] = make_float2(o4[2], o4[3]);
             ao[i][0] = ao[i][1] = make_float2(0.f, 0.f);
           }
 #pragma unroll 2
@@ -792,7 +874,10 @@ __global__ void __launch_bounds__(256) adjoint_pipe_kernel(
             float xv[4];
             Pipe<DT>::chunk4(buf + (size_t)j * L.RS + 4 * q * EB, xv);
             const float2 x01 = make_float2(xv[0], xv[1]), x23 = make_float2(xv[2], xv[3]);
-            const float* cj = coef + (size_t)j * L.CS;
+            float cj[(OMX + 3) & ~3];
+#pragma unroll
+            for (int i = 0; i < OMX; i += 4)
+              lds4(coef + (size_t)j * L.CS + i, *reinterpret_cast<float(*)[4]>(cj + i));
             float2 a01 = make_float2(0.f, 0.f), a23 = a01;
 #pragma unroll
             for (int i = 0; i < OMX; i++) {
@@ -803,13 +888,13 @@ __global__ void __launch_bounds__(256) adjoint_pipe_kernel(
               ao[i][1] = __ffma2_rn(c2, x23, ao[i][1]);
             }
             const float ai[4] = {a01.x, a01.y, a23.x, a23.y};
-            atomic_add4(g_in + (size_t)slot[j] * d + 4 * q, ai);
+            add_row4(g_in, slot[j], d, q, ai);
           }
 #pragma unroll
           for (int i = 0; i < OMX; i++)
             if (i < O) {
               const float v[4] = {ao[i][0].x, ao[i][0].y, ao[i][1].x, ao[i][1].y};
-              atomic_add4(g_out + (size_t)slot[I + i] * d + 4 * q, v);
+              add_row4(g_out, slot[I + i], d, q, v);
             }
         }
       }
@@ -831,6 +916,19 @@ __global__ void __launch_bounds__(256) adjoint_pipe_kernel(
   cp_async_wait_all();
   for (int sh = 16; sh > 0; sh >>= 1) loss += __shfl_xor_sync(kFull, loss, sh);
   if (lane == 0 && loss != 0) atomicAdd(&loss_parts[gw & 255], (double)loss);
+  // the last block to get here adds up the partial sums
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(&info[INFO_DONE], 1) == (int)gridDim.x - 1;
+  __syncthreads();
+  if (last && threadIdx.x < 32) {
+    __threadfence();
+    double v = 0;
+    for (int k = lane; k < 256; k += 32) v += __ldcg(&loss_parts[k]);
+    for (int sh = 16; sh > 0; sh >>= 1) v += __shfl_xor_sync(kFull, v, sh);
+    if (lane == 0) *loss_out = v;
+  }
 }
 
 __global__ void finish_loss_kernel(const double* parts, double* loss) {
@@ -846,63 +944,61 @@ __global__ void finish_loss_kernel(const double* parts, double* loss) {
   }
 }
 
-void scan_and_emit(int32_t* a, int64_t V, int32_t* tile_sums, int32_t* ids, cudaStream_t s) {
-  const int64_t tiles = (V + kScanTile - 1) / kScanTile;
-  scan_tiles_kernel<<<(unsigned)tiles, kScanThreads, 0, s>>>(a, V, tile_sums);
-  scan_tile_sums_kernel<<<1, kScanThreads, 0, s>>>(tile_sums, tiles);
-  const unsigned g = (unsigned)std::min<int64_t>((V + 255) / 256, 152 * 32);
-  add_prefix_emit_kernel<<<g, 256, 0, s>>>(a, V, tile_sums, ids);
-  add_prefix_kernel<<<g, 256, 0, s>>>(a, V, tile_sums);
+// A call's scratch: info words, 256 fp64 loss sums, the marks of both tables (cleared
+// together), then the tiles' counts.
+struct AdjointScratch {
+  int32_t* info;
+  double* loss_parts;
+  RowMark* marks;  // input table, then output table
+  int32_t* sums;
+  int64_t words, tiles;
+  size_t cleared, bytes;
+};
+AdjointScratch adjoint_scratch(void* base, int64_t V) {
+  AdjointScratch a;
+  char* p = static_cast<char*>(base);
+  a.words = (V + 31) / 32;
+  a.tiles = (a.words + kMarkTile - 1) / kMarkTile;
+  a.info = reinterpret_cast<int32_t*>(p);
+  a.loss_parts = reinterpret_cast<double*>(p + 64);
+  a.marks = reinterpret_cast<RowMark*>(p + 64 + 256 * sizeof(double));
+  a.cleared = 64 + 256 * sizeof(double) + 2 * (size_t)a.words * sizeof(RowMark);
+  a.sums = reinterpret_cast<int32_t*>(p + a.cleared);
+  a.bytes = a.cleared + 2 * (size_t)a.tiles * sizeof(int32_t);
+  return a;
 }
 
 }  // namespace
 
-size_t adjoint_scratch_bytes(int64_t V) {
-  const int64_t tiles = (V + kScanTile - 1) / kScanTile;
-  // marks (2V), tile sums, status words, then 256 fp64 loss partials (8-byte aligned)
-  return sizeof(int32_t) * (size_t)(2 * V + 2 * tiles + 8) + 8 + 256 * sizeof(double);
-}
-double* loss_parts_of(void* scratch, int64_t V) {
-  const int64_t tiles = (V + kScanTile - 1) / kScanTile;
-  const size_t off = (sizeof(int32_t) * (size_t)(2 * V + 2 * tiles + 8) + 7) & ~(size_t)7;
-  return reinterpret_cast<double*>(static_cast<char*>(scratch) + off);
-}
+size_t adjoint_scratch_bytes(int64_t V) { return adjoint_scratch(nullptr, V).bytes; }
 
-// Phase 1: marks, checks, the row -> slot prefix sums, the emitted ids and the zeroed
-// gradient rows.  info[0..1] = distinct input / output rows, info[2] = status bits,
-// info[3..4] = the largest input / output count of a minibatch (device memory; the host
-// reads them before phase 2).  scratch: adjoint_scratch_bytes(V) bytes, arbitrary on entry.
+// Phase 1: marks, checks, slots, the emitted ids and the zeroed gradient rows.  *info_out
+// (device, in scratch): distinct input rows, distinct output rows, status bits, the largest
+// input and output count of a minibatch; the host reads them before phase 2.  scratch:
+// adjoint_scratch_bytes(V) bytes, 16-byte aligned, arbitrary on entry.
 cudaError_t launch_adjoint_prepare(int dtype, int d, int n, int64_t V, const int32_t* in_ptr, const int32_t* in_ids,
                                    const int32_t* in_first, const int32_t* out_ptr, const int32_t* out_ids,
                                    double* loss, int32_t* grad_in_ids, void* grad_in, int32_t* grad_out_ids,
-                                   void* grad_out, int32_t* info, void* scratch, cudaStream_t s) {
-  const int64_t tiles = (V + kScanTile - 1) / kScanTile;
-  int32_t* incl_in = static_cast<int32_t*>(scratch);
-  int32_t* incl_out = incl_in + V;
-  int32_t* sums_in = incl_out + V;
-  int32_t* sums_out = sums_in + tiles;
-  int32_t* status = sums_out + tiles;  // status, imax, omax
+                                   void* grad_out, const int32_t** info_out, void* scratch, cudaStream_t s) {
+  const AdjointScratch a = adjoint_scratch(scratch, V);
+  *info_out = a.info;
   cudaError_t e;
-  if ((e = cudaMemsetAsync(incl_in, 0, sizeof(int32_t) * 2 * V, s)) != cudaSuccess) return e;
-  if ((e = cudaMemsetAsync(status, 0, sizeof(int32_t) * 3, s)) != cudaSuccess) return e;
-  if ((e = cudaMemsetAsync(loss, 0, sizeof(double), s)) != cudaSuccess) return e;
-  if ((e = cudaMemsetAsync(loss_parts_of(scratch, V), 0, 256 * sizeof(double), s)) != cudaSuccess) return e;
-  if (n > 0)
-    mark_rows_kernel<<<(unsigned)std::min<int64_t>(((int64_t)n + 7) / 8, 152 * 16), 256, 0, s>>>(
-        n, in_ptr, in_ids, in_first, out_ptr, out_ids, V, incl_in, incl_out, status, status + 1);
-  scan_and_emit(incl_in, V, sums_in, grad_in_ids, s);
-  scan_and_emit(incl_out, V, sums_out, grad_out_ids, s);
-  const unsigned zg = 152 * 16;
-  if (dtype == 2) {
-    zero_rows_kernel<double><<<zg, 256, 0, s>>>(static_cast<double*>(grad_in), incl_in + V - 1, d);
-    zero_rows_kernel<double><<<zg, 256, 0, s>>>(static_cast<double*>(grad_out), incl_out + V - 1, d);
-  } else {
-    zero_rows_kernel<float><<<zg, 256, 0, s>>>(static_cast<float*>(grad_in), incl_in + V - 1, d);
-    zero_rows_kernel<float><<<zg, 256, 0, s>>>(static_cast<float*>(grad_out), incl_out + V - 1, d);
-  }
-  if ((e = cudaMemcpyAsync(info, incl_in + V - 1, sizeof(int32_t), cudaMemcpyDeviceToDevice, s))) return e;
-  if ((e = cudaMemcpyAsync(info + 1, incl_out + V - 1, sizeof(int32_t), cudaMemcpyDeviceToDevice, s))) return e;
-  if ((e = cudaMemcpyAsync(info + 2, status, sizeof(int32_t) * 3, cudaMemcpyDeviceToDevice, s))) return e;
+  if ((e = cudaMemsetAsync(scratch, 0, a.cleared, s)) != cudaSuccess) return e;
+  if (n <= 0) return cudaMemsetAsync(loss, 0, sizeof(double), s);
+  RowMark* mark_out = a.marks + a.words;
+  mark_rows_kernel<<<(unsigned)std::min<int64_t>(((int64_t)n + 15) / 16, 152 * 4), kHotThreads, 0, s>>>(
+      n, in_ptr, in_ids, in_first, out_ptr, out_ids, V, a.marks, mark_out, a.info);
+  const dim3 tiles((unsigned)a.tiles, 2);
+  count_tiles_kernel<<<tiles, kMarkThreads, 0, s>>>(a.marks, a.words, a.sums, (int)a.tiles);
+  emit_rows_kernel<<<tiles, kMarkThreads, 0, s>>>(a.marks, a.words, a.sums, (int)a.tiles, grad_in_ids, grad_out_ids,
+                                                  a.info);
+  const unsigned zg = (unsigned)std::min<int64_t>((2 * a.words + 7) / 8, 152 * 16);
+  if (dtype == 2)
+    zero_rows_kernel<double><<<zg, 256, 0, s>>>(a.marks, a.words, static_cast<double*>(grad_in),
+                                                static_cast<double*>(grad_out), d);
+  else
+    zero_rows_kernel<float><<<zg, 256, 0, s>>>(a.marks, a.words, static_cast<float*>(grad_in),
+                                               static_cast<float*>(grad_out), d);
   return cudaGetLastError();
 }
 
@@ -920,9 +1016,9 @@ cudaError_t launch_adjoint(int dtype, int d, int n, int64_t V, int imax, int oma
                            const int32_t* out_ids, const int32_t* out_meta, const void* wih, const void* woh,
                            double* loss, void* grad_in, void* grad_out, void* scratch, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  double* parts = loss_parts_of(scratch, V);
-  const int32_t* incl_in = static_cast<const int32_t*>(scratch);
-  const int32_t* incl_out = incl_in + V;
+  const AdjointScratch a = adjoint_scratch(scratch, V);
+  double* parts = a.loss_parts;
+  const RowMark *mark_in = a.marks, *mark_out = a.marks + a.words;
   imax = std::max(imax, 1);
   omax = std::max(omax, 1);
   const int wpb = adjoint_warps_per_block(dtype, d, imax, omax);
@@ -935,7 +1031,7 @@ cudaError_t launch_adjoint(int dtype, int d, int n, int64_t V, int imax, int oma
                                   (int)smem)))                                                                  \
       return e;                                                                                                 \
     adjoint_kernel<DT, VW, OMX><<<blocks, 32 * wpb, smem, s>>>(                                                 \
-        d, n, imax, omax, in_ptr, in_ids, in_first, out_ptr, out_ids, out_meta, wih, woh, V, incl_in, incl_out, \
+        d, n, imax, omax, in_ptr, in_ids, in_first, out_ptr, out_ids, out_meta, wih, woh, V, mark_in, mark_out, \
         static_cast<TT*>(grad_in), static_cast<TT*>(grad_out), parts);                                          \
   } while (0)
 #define SGNS_ADJ_LAUNCH(DT, VW, TT)                   \
@@ -950,13 +1046,13 @@ cudaError_t launch_adjoint(int dtype, int d, int n, int64_t V, int imax, int oma
   const int ring = imax + omax;
   const PipeLayout PL = pipe_layout(dtype, d, imax, omax, omax <= 7 ? 7 : kOMax, ring);
   if (v4 && (d * eb) % 16 == 0 && ((uintptr_t)wih & 15) == 0 && ((uintptr_t)woh & 15) == 0 &&
-      PL.bytes <= 232448) {
+      PL.bytes <= kPipeSmem) {
     // warps per block: the most resident warps per SM (228 KB of shared memory, 1 KB
     // reserved per block), the larger block on a tie
     int pw = 1, best = 0;
     for (int w = 1; w <= 8; w++) {
-      const int per_block = w * PL.bytes + 1024;
-      if (w * PL.bytes > 232448) break;
+      const int per_block = w * PL.bytes + 1024 + 64;
+      if (w * PL.bytes > kPipeSmem) break;
       const int warps = (233472 / per_block) * w;
       if (warps >= best) best = warps, pw = w;
     }
@@ -975,9 +1071,9 @@ cudaError_t launch_adjoint(int dtype, int d, int n, int64_t V, int imax, int oma
     const unsigned pb = (unsigned)std::max<int64_t>(                                                            \
         1, std::min<int64_t>((n + pw - 1) / pw, (int64_t)sms * std::max(per_sm, 1)));                           \
     adjoint_pipe_kernel<DT, OMX><<<pb, 32 * pw, psmem, s>>>(d, n, imax, omax, ring, in_ptr, in_ids, in_first, out_ptr, \
-                                                            out_ids, out_meta, wih, woh, V, incl_in, incl_out,   \
+                                                            out_ids, out_meta, wih, woh, V, mark_in, mark_out,   \
                                                             static_cast<TT*>(grad_in),                          \
-                                                            static_cast<TT*>(grad_out), parts);                 \
+                                                            static_cast<TT*>(grad_out), parts, a.info, loss);   \
   } while (0)
 #define SGNS_ADJ_PIPE(DT, TT)                  \
   do {                                         \
@@ -989,7 +1085,6 @@ cudaError_t launch_adjoint(int dtype, int d, int n, int64_t V, int imax, int oma
     else SGNS_ADJ_PIPE(0, float);
 #undef SGNS_ADJ_PIPE
 #undef SGNS_ADJ_PIPE1
-    finish_loss_kernel<<<1, 256, 0, s>>>(parts, loss);
     return cudaGetLastError();
   }
   if (dtype == 2) {

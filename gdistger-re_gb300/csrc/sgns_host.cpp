@@ -395,7 +395,28 @@ sgns_status finish_stats(sgns_handle* h, int workers, float ms) {
   return SGNS_OK;
 }
 
-// largest worker count the persistent engine keeps resident in one wave
+// Default worker count of wpc workers per CTA.  The count decides every worker's corpus slice
+// and random streams, so it is a fixed rule of the problem's sizes and not of the kernels'
+// present footprint: the one-warp workers that an SM holds (8 warps, 228 KB of shared memory)
+// with 2w + 2 padded rows per walk, the output rows, gradient pairs and both walks in flight.
+int rule_workers(const sgns_handle* h, int wpc) {
+  const sgns_options& o = h->opt;
+  const int64_t om = o.negative <= 5 ? 7 : kOMax, op = (om + 1) & ~1LL, im = 4 * o.window, row = o.size + 4;
+  const int64_t words = 2 * (2 * o.window + 2) * row + op * row + im * (op + 2) * 2 + 2 * (int64_t)h->lmax + im + 2 * om +
+                        2 * (o.window + 1);
+  const int64_t smem = 4 * (1136 + wpc * ((words + 3) & ~3LL));
+  if (smem > 232448) return 0;
+  const int64_t ctas = std::min<int64_t>(233472 / (smem + 1024), 8 / wpc);
+  // At most V/400 workers: with many workers per vertex in flight, hot rows are updated
+  // from many stale window copies at once, which costs link-prediction quality (4-block
+  // SBM, 100k vertices, every worker in flight: AUC 0.7865 with 266 workers, 0.7842 with
+  // 532, 0.7804 with 1064, against the reference trainer's 0.7886).  Large vocabularies
+  // keep the full resident count (2.24M vertices: 5596 > 1064).
+  return (int)std::min<int64_t>(ctas * wpc * h->num_sms, std::max<int64_t>(1, h->V / 400));
+}
+
+// Whether the persistent engine's present shape (team or one warp, wpc workers per CTA) can
+// run, and its default worker count.
 sgns_status persistent_shape(sgns_handle* h, int wpc, int* workers) {
   int ctas = 0;
   const sgns_options& o = h->opt;
@@ -407,14 +428,9 @@ sgns_status persistent_shape(sgns_handle* h, int wpc, int* workers) {
   if (ctas < 1)
     return fail(h, SGNS_EINVAL, "a %d-warp CTA does not fit in shared memory (d=%d, walks up to %d)", wpc,
                 o.size, h->lmax);
-  *workers = ctas * wpc * h->num_sms;
-  // At most V/400 workers: with many workers per vertex in flight, hot rows are updated
-  // from many stale window copies at once, which costs link-prediction quality (4-block
-  // SBM, 100k vertices, every worker in flight: AUC 0.7865 with 266 workers, 0.7842 with
-  // 532, 0.7804 with 1064, against the reference trainer's 0.7886).  Large vocabularies
-  // keep the full resident count (2.24M vertices: 5596 > 1064).
-  const int64_t cap = std::max<int64_t>(1, h->V / 400);
-  if (*workers > cap) *workers = (int)cap;
+  *workers = rule_workers(h, wpc);
+  if (*workers < 1)  // fits only as the kernels are now
+    *workers = (int)std::min<int64_t>((int64_t)ctas * wpc * h->num_sms, std::max<int64_t>(1, h->V / 400));
   return SGNS_OK;
 }
 
@@ -583,6 +599,8 @@ void shape_for_wpc(sgns_handle* h, int wpc) {
 sgns_status autotune(sgns_handle* h) {
   const sgns_options& o = h->opt;
   const std::string key = tune_key(h);
+  int rule = 0;  // the default worker count: the most that any CTA shape's rule gives
+  for (int wpc = 1; wpc <= 8; wpc++) rule = std::max(rule, rule_workers(h, wpc));
   auto use = [&](const Shape& c) {
     h->team = c.team;
     h->tile = c.tile;
@@ -596,7 +614,7 @@ sgns_status autotune(sgns_handle* h) {
       use(c);
       int workers = 0;
       if (persistent_shape(h, c.wpc, &workers) == SGNS_OK) {
-        h->workers = o.workers > 0 ? o.workers : workers;
+        h->workers = o.workers > 0 ? o.workers : rule > 0 ? rule : workers;
         h->tuned = true;
         if (o.debug > 0)
           fprintf(stderr, "sgns: persistent engine shape from the tuning cache: %d workers/CTA, tile %d, team %d\n", c.wpc,
@@ -648,20 +666,20 @@ sgns_status autotune(sgns_handle* h) {
   sgns_status st = SGNS_OK;
   cudaError_t e;
   if ((e = cudaMalloc(&wih_s, tbytes)) != cudaSuccess || (e = cudaMalloc(&woh_s, tbytes)) != cudaSuccess) {
-    // no room for scratch tables: take, untimed, the shape with the most resident
-    // workers; ties go to the first (teams before single warps, small CTAs before large ones)
+    // no room for scratch tables: untimed, the one-warp shape with the most workers (a warp
+    // each fills the GPU best), or what fits
     restore();
     cudaGetLastError();
     for (const Shape& c : shapes) {
       int workers = 0;
       use(c);
-      if (persistent_shape(h, c.wpc, &workers) == SGNS_OK && workers > best_workers) {
+      if (persistent_shape(h, c.wpc, &workers) == SGNS_OK && (workers > best_workers || (best_shape.team && !c.team))) {
         best_shape = c;
         best_workers = workers;
       }
     }
     use(best_shape);
-    h->workers = o.workers > 0 ? o.workers : best_workers;
+    h->workers = o.workers > 0 ? o.workers : rule > 0 ? rule : best_workers;
     h->tuned = true;
     if (o.debug > 0)
       fprintf(stderr, "sgns: no memory for autotuning; persistent engine at %d warps/CTA\n", best_shape.wpc);
@@ -681,6 +699,7 @@ sgns_status autotune(sgns_handle* h) {
     st = persistent_shape(h, c.wpc, &workers);
     if (st) break;
     if (o.workers > 0) workers = o.workers;
+    else if (rule > 0) workers = rule;
     // a prefix long enough to give every worker a few hundred steps
     h->n_tokens = std::min<int64_t>(n0, (int64_t)workers * 2000);
     float ms = 0.f;
@@ -1628,13 +1647,13 @@ sgns_status sgns_loss_adjoint(int32_t dtype, int32_t d, int64_t V, int32_t n, co
   DeviceScratch* ds = device_scratch();
   if (!ds) return fail(nullptr, SGNS_ECUDA, "no current CUDA device");
   std::lock_guard<std::mutex> g(ds->mx);
-  sgns_status st = ds->ensure(adjoint_scratch_bytes(V) + 64);
+  sgns_status st = ds->ensure(adjoint_scratch_bytes(V));
   if (st) return st;
-  int32_t* info = reinterpret_cast<int32_t*>(static_cast<char*>(ds->buf) + adjoint_scratch_bytes(V));
+  const int32_t* info = nullptr;
   // phase 1 finds, on the device, the distinct rows and the largest minibatch; its sizes
   // (five ints) are the one read-back before the gradient kernel
   cudaError_t e = launch_adjoint_prepare(dtype, d, n, V, in_ptr, in_ids, in_first, out_ptr, out_ids, loss,
-                                         grad_in_ids, grad_in, grad_out_ids, grad_out, info, ds->buf, s);
+                                         grad_in_ids, grad_in, grad_out_ids, grad_out, &info, ds->buf, s);
   int32_t h[5];
   if (e == cudaSuccess) e = cudaMemcpyAsync(h, info, sizeof h, cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);

@@ -250,13 +250,13 @@ void host_exp_table(float* t /* kExpTableSize + 1 */);
 int report_error(int status, const char* fmt, ...);  // sets sgns_last_error(NULL); returns status
 
 size_t adjoint_scratch_bytes(int64_t V);
-// phase 1 of the adjoint: marks, checks, slots, ids, zeroed gradient rows; info (device, 5
-// ints): distinct input rows, distinct output rows, status bits (1 bad id, 2 bad size),
-// largest input count, largest output count
+// phase 1 of the adjoint: marks, checks, slots, ids, zeroed gradient rows; *info (device, 5
+// ints in scratch): distinct input rows, distinct output rows, status bits (1 bad id, 2 bad
+// size), largest input count, largest output count
 cudaError_t launch_adjoint_prepare(int dtype, int d, int n, int64_t V, const int32_t* in_ptr, const int32_t* in_ids,
                                    const int32_t* in_first, const int32_t* out_ptr, const int32_t* out_ids,
                                    double* loss, int32_t* grad_in_ids, void* grad_in, int32_t* grad_out_ids,
-                                   void* grad_out, int32_t* info, void* scratch, cudaStream_t s);
+                                   void* grad_out, const int32_t** info, void* scratch, cudaStream_t s);
 // phase 2: loss and row gradients (imax / omax from phase 1)
 cudaError_t launch_adjoint(int dtype, int d, int n, int64_t V, int imax, int omax, const int32_t* in_ptr,
                            const int32_t* in_ids, const int32_t* in_first, const int32_t* out_ptr,
