@@ -1306,7 +1306,7 @@ sgns_status parse_walks(sgns_handle* h, const uint8_t* bytes, int64_t n, int32_t
   long long err = 0, mx = -1;
   cudaError_t e = launch_ingest_count(bytes, n, ds->buf, &cnt, &err, s);
   if (e != cudaSuccess) return fail(h, SGNS_ECUDA, "walk parse: %s", cudaGetErrorString(e));
-  if (err != 0x7FFFFFFFFFFFFFFFLL) {
+  if (err != kIngestNoError) {
     uint8_t c = 0;
     cudaMemcpy(&c, bytes + err, 1, cudaMemcpyDeviceToHost);
     return fail(h, SGNS_EINVAL, "unexpected byte 0x%02x at offset %lld of the walk text", c, err);
@@ -1318,7 +1318,7 @@ sgns_status parse_walks(sgns_handle* h, const uint8_t* bytes, int64_t n, int32_t
   if (cnt == 0) return SGNS_OK;
   e = launch_ingest_emit(bytes, n, ds->buf, tokens, &err, &mx, s);
   if (e != cudaSuccess) return fail(h, SGNS_ECUDA, "walk parse: %s", cudaGetErrorString(e));
-  if (err != 0x7FFFFFFFFFFFFFFFLL)
+  if (err != kIngestNoError)
     return fail(h, SGNS_EINVAL, "vertex id ending at offset %lld of the walk text exceeds 2^31 - 1", err);
   *max_id = mx;
   return SGNS_OK;

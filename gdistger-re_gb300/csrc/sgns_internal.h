@@ -218,6 +218,7 @@ cudaError_t launch_minibatch_bf16(int d, int n, int imax, const int32_t* in_coun
 // host helpers shared by the translation units (sgns_host.cpp)
 // walk-file text -> corpus (dsgl_ingest.cu); scratch of ingest_scratch_bytes(n) bytes
 size_t ingest_scratch_bytes(int64_t n);
+constexpr long long kIngestNoError = 0x7F7F7F7F7F7F7F7FLL;  // *err_pos when no byte is at fault
 cudaError_t launch_ingest_count(const uint8_t* bytes, int64_t n, void* scratch, unsigned long long* n_out,
                                 long long* err_pos, cudaStream_t s);
 cudaError_t launch_ingest_emit(const uint8_t* bytes, int64_t n, void* scratch, int32_t* tokens, long long* err_pos,
