@@ -65,7 +65,8 @@ __global__ void map_corpus_kernel(const int32_t* ids, const int32_t* row_of, int
 // What bounds it: the chains' latency (a dot product is d dependent multiply-adds) at the five
 // blocks that 43 KB of rows (64 inputs, d = 128) leave per SM.  20,000 minibatches of 19.6
 // inputs, d = 128, rounded write-back: 2,260 us with one warp per minibatch, the sigmoid table
-// copied to shared memory per block and a one-thread prefix of the counts; 142 us now.
+// copied to shared memory per block and a one-thread prefix of the counts; 297 us now
+// (60 us of bytes).
 constexpr int kMbThreads = 128;
 constexpr int kMbOwnPrefix = 1024;  // up to here a block sums the counts before its own itself
 

@@ -49,6 +49,9 @@ template <> struct RowIO<STORE_F32> {
   __device__ static __forceinline__ Raw load_raw(const void* base, int64_t row, int d, int q) {
     return reinterpret_cast<const float4*>(static_cast<const float*>(base) + row * d)[q];
   }
+  __device__ static __forceinline__ Raw load_l2(const void* base, int64_t row, int d, int q) {  // past the L1
+    return __ldcg(reinterpret_cast<const float4*>(static_cast<const float*>(base) + row * d) + q);
+  }
   __device__ static __forceinline__ float4 widen(Raw r) { return r; }
   __device__ static __forceinline__ float4 load4(const void* base, int64_t row, int d, int q) {
     return reinterpret_cast<const float4*>(static_cast<const float*>(base) + row * d)[q];
@@ -65,6 +68,9 @@ template <> struct RowIO<STORE_BF16> {
   typedef uint2 Raw;
   __device__ static __forceinline__ Raw load_raw(const void* base, int64_t row, int d, int q) {
     return reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(base) + row * d)[q];
+  }
+  __device__ static __forceinline__ Raw load_l2(const void* base, int64_t row, int d, int q) {  // past the L1
+    return __ldcg(reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(base) + row * d) + q);
   }
   __device__ static __forceinline__ float4 widen(Raw u) {
     return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xFFFF0000u),
