@@ -22,6 +22,9 @@
 // shared memory returns to the registers.  The register tiles read a third of the bytes that
 // one lane per input did, and the gradients are kept once instead of as pairs: 1.1M vertices,
 // 1064 workers, d = 128: bf16 182.3 -> 159.7 ms a pass, d = 64 21.2 -> 16.7 (400k vertices).
+// Table rows are read past the L1 (load_l2): a line there can be older than what another SM's
+// worker has stored, and would be written back as it was (100k vertices, 250 workers: AUC
+// 0.7764 -> 0.7770 in bf16, 0.7779 -> 0.7786 in fp32; pass times are the same).
 // A compact loop matters as much: batching or prefetching the backward's inputs four deep
 // cost 4-9% in instruction fetch.  The negative pool keeps the reference's
 // draw stream (max(len1,len2)*K draws per pool, group neg_count % n per step,
@@ -91,7 +94,7 @@ __device__ __forceinline__ void load_rows_batched(const void* tab, const int* id
 #pragma unroll
         for (int t = 0; t < DCH; t++) {
           const int q = lane + 32 * t;
-          if (q < d4) v[u][t] = RowIO<S>::load4(tab, row, d, q);
+          if (q < d4) v[u][t] = RowIO<S>::widen(RowIO<S>::load_l2(tab, row, d, q));
         }
       }
     }
@@ -346,7 +349,7 @@ __global__ void __launch_bounds__(256) window_engine_kernel(TrainParams p) {
 #pragma unroll
         for (int t = 0; t < DCH; t++) {
           const int q = lane + 32 * t;
-          ov[i][t] = (i < O && q < d4) ? RowIO<S>::load_raw(p.woh, row, d, q) : typename RowIO<S>::Raw{};
+          ov[i][t] = (i < O && q < d4) ? RowIO<S>::load_l2(p.woh, row, d, q) : typename RowIO<S>::Raw{};
         }
       }
     }
@@ -472,7 +475,7 @@ __global__ void __launch_bounds__(256) window_engine_kernel(TrainParams p) {
 #pragma unroll
         for (int t = 0; t < DCH; t++) {
           const int q = lane + 32 * t;
-          ov[i][t] = (i < O_next && q < d4) ? RowIO<S>::load_raw(p.woh, row, d, q) : typename RowIO<S>::Raw{};
+          ov[i][t] = (i < O_next && q < d4) ? RowIO<S>::load_l2(p.woh, row, d, q) : typename RowIO<S>::Raw{};
         }
       }
       ov_ready = true;
@@ -520,7 +523,7 @@ __global__ void __launch_bounds__(256) window_engine_kernel(TrainParams p) {
             if (fresh) {
 #pragma unroll
               for (int t = 0; t < DCH; t++)
-                if (lane + 32 * t < d4) ent[walk][t] = RowIO<S>::load_raw(p.wih, v, d, lane + 32 * t);
+                if (lane + 32 * t < d4) ent[walk][t] = RowIO<S>::load_l2(p.wih, v, d, lane + 32 * t);
               ent_off[walk] = (walk * NS + s) * DP;
               n_loads++;
             }
