@@ -415,9 +415,9 @@ int rule_workers(const sgns_handle* h, int wpc) {
   return (int)std::min<int64_t>(ctas * wpc * h->num_sms, std::max<int64_t>(1, h->V / 400));
 }
 
-// Whether the persistent engine's present shape (team or one warp, wpc workers per CTA) can
-// run, and its default worker count.
-sgns_status persistent_shape(sgns_handle* h, int wpc, int* workers) {
+// Workers of the persistent engine's present shape (team or one warp, wpc workers per CTA)
+// that the GPU holds at once; 0 when a CTA does not fit.
+sgns_status resident_workers(sgns_handle* h, int wpc, int64_t* resident) {
   int ctas = 0;
   const sgns_options& o = h->opt;
   const int storage = o.storage == SGNS_STORE_BF16_SR ? STORE_BF16 : STORE_F32;
@@ -425,12 +425,21 @@ sgns_status persistent_shape(sgns_handle* h, int wpc, int* workers) {
     CU(h, team_engine_occupancy(storage, o.size, o.window, o.negative, h->lmax, wpc, &ctas));
   else
     CU(h, window_engine_occupancy(storage, o.size, o.window, o.negative, h->lmax, wpc, &ctas));
-  if (ctas < 1)
+  *resident = (int64_t)ctas * wpc * h->num_sms;
+  return SGNS_OK;
+}
+
+// Whether the present shape can run, and its default worker count.
+sgns_status persistent_shape(sgns_handle* h, int wpc, int* workers) {
+  int64_t resident = 0;
+  sgns_status st = resident_workers(h, wpc, &resident);
+  if (st) return st;
+  if (resident < 1)
     return fail(h, SGNS_EINVAL, "a %d-warp CTA does not fit in shared memory (d=%d, walks up to %d)", wpc,
-                o.size, h->lmax);
+                h->opt.size, h->lmax);
   *workers = rule_workers(h, wpc);
   if (*workers < 1)  // fits only as the kernels are now
-    *workers = (int)std::min<int64_t>((int64_t)ctas * wpc * h->num_sms, std::max<int64_t>(1, h->V / 400));
+    *workers = (int)std::min<int64_t>(resident, std::max<int64_t>(1, h->V / 400));
   return SGNS_OK;
 }
 
@@ -590,9 +599,9 @@ void shape_for_wpc(sgns_handle* h, int wpc) {
 
 // Autotuner: times launch shapes of the persistent engine on a prefix of the corpus, on
 // scratch copies of the tables, and keeps the fastest (pairs per second).  Where teams may
-// train the workers: a team per worker at 1, 2 and 3 workers per CTA (few workers spread best
-// in small CTAs) and one warp per worker at 4..8 (the shapes that fill an SM); else one warp
-// per worker at 1..8.
+// train the workers and an SM holds as many as it gets: a team per worker at 1, 2 and 3 workers
+// per CTA (few workers spread best in small CTAs) and one warp per worker at 4..8 (the shapes
+// that fill an SM); else one warp per worker at 1..8.
 // Autotuner cache: with SGNS_TUNE_CACHE naming a file, the choice is kept per device model
 // and problem shape and reused by later runs.  The file is only an optimisation: any error
 // reading or writing it is ignored.
@@ -606,23 +615,6 @@ sgns_status autotune(sgns_handle* h) {
     h->tile = c.tile;
     h->wpc = c.wpc;
   };
-  if (o.warps_per_cta <= 0) {
-    Shape c{};
-    if (tune_cache_lookup(key, &c) && (!c.team || teams_allowed(o))) {
-      if (!window_engine_has_tile2(o.size, o.negative)) c.tile = 1;
-      if (o.forward_tile > 0) c.tile = o.forward_tile;
-      use(c);
-      int workers = 0;
-      if (persistent_shape(h, c.wpc, &workers) == SGNS_OK) {
-        h->workers = o.workers > 0 ? o.workers : rule > 0 ? rule : workers;
-        h->tuned = true;
-        if (o.debug > 0)
-          fprintf(stderr, "sgns: persistent engine shape from the tuning cache: %d workers/CTA, tile %d, team %d\n", c.wpc,
-                  c.tile, (int)c.team);
-        return SGNS_OK;
-      }
-    }
-  }
   if (o.warps_per_cta > 0) {  // a given CTA shape
     h->wpc = o.warps_per_cta;
     shape_for_wpc(h, h->wpc);
@@ -634,16 +626,44 @@ sgns_status autotune(sgns_handle* h) {
     h->tuned = true;
     return SGNS_OK;
   }
+  // Shapes that hold all the workers at once.  The reference's threads run side by side over
+  // their slices (dsgl.hpp:783-826) under one learning rate; a worker that waits for another
+  // to end trains its whole slice at the schedule's low end, and a last wave of few workers
+  // takes as long as a full one.  When no shape holds a given count, one warp per worker does
+  // as many at once as fit.
+  const int want = o.workers > 0 ? o.workers : rule;
   std::vector<Shape> shapes;
-  auto consider = [&](const Shape& c) {
-    int workers = 0;
+  auto holds = [&](const Shape& c, int64_t n) {
+    int64_t resident = 0;
     use(c);
-    if (persistent_shape(h, c.wpc, &workers) == SGNS_OK) shapes.push_back(c);
+    return resident_workers(h, c.wpc, &resident) == SGNS_OK && resident >= std::max<int64_t>(n, 1);
+  };
+  auto consider = [&](const Shape& c, int64_t n) {
+    if (holds(c, n)) shapes.push_back(c);
   };
   if (teams_allowed(o))
-    for (int wpc = 1; wpc <= kTeamMaxPerCta; wpc++) consider(Shape{true, wpc, 1});
-  for (int wpc = shapes.empty() ? 1 : 4; wpc <= 8; wpc++) consider(Shape{false, wpc, default_tile(h)});
+    for (int wpc = 1; wpc <= kTeamMaxPerCta; wpc++) consider(Shape{true, wpc, 1}, want);
+  for (int wpc = shapes.empty() ? 1 : 4; wpc <= 8; wpc++) consider(Shape{false, wpc, default_tile(h)}, want);
+  const bool all_held = !shapes.empty();
+  if (!all_held)
+    for (int wpc = 1; wpc <= 8; wpc++) consider(Shape{false, wpc, default_tile(h)}, 1);
   if (shapes.empty()) return fail(h, SGNS_EINVAL, "no persistent-engine shape fits this configuration");
+  Shape cached{};
+  if (tune_cache_lookup(key, &cached) && (!cached.team || teams_allowed(o)) &&
+      holds(cached, all_held || cached.team ? want : 1)) {
+    if (!window_engine_has_tile2(o.size, o.negative)) cached.tile = 1;
+    if (o.forward_tile > 0) cached.tile = o.forward_tile;
+    use(cached);
+    int workers = 0;
+    if (persistent_shape(h, cached.wpc, &workers) == SGNS_OK) {
+      h->workers = o.workers > 0 ? o.workers : rule > 0 ? rule : workers;
+      h->tuned = true;
+      if (o.debug > 0)
+        fprintf(stderr, "sgns: persistent engine shape from the tuning cache: %d workers/CTA, tile %d, team %d\n",
+                cached.wpc, cached.tile, (int)cached.team);
+      return SGNS_OK;
+    }
+  }
   // the trial launches train scratch copies of the tables; the handle's own pointers,
   // corpus length and pass count are put back on every path out of the search
   const size_t tbytes = (size_t)h->V * o.size * elem_bytes(o);

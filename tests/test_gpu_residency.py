@@ -1,0 +1,49 @@
+"""Workers that a launch of the persistent engine holds at once.
+
+The reference's compute threads run side by side (dsgl.hpp:783-826, one slice each) under one
+learning-rate schedule, so a launch shape must hold all the workers of a call: a worker that
+starts when another has ended trains its whole slice at the low end of the schedule.  An SM
+holds at most three teams (128 registers x 160 threads each) and eight one-warp workers (up
+to 255 registers a thread), in whole CTAs."""
+import re
+
+import numpy as np
+import pytest
+
+import sgns
+
+pytestmark = pytest.mark.gpu
+
+
+def small_corpus(V, n_walks, seed):
+    rng = np.random.default_rng(seed)
+    walks = np.hstack([rng.integers(0, V, (n_walks, 30)), -np.ones((n_walks, 1), np.int64)]).ravel().astype(np.int32)
+    return walks, np.maximum(np.bincount(walks[walks >= 0], minlength=V), 1).astype(np.int32)
+
+
+def held(team, per_cta):
+    import torch
+
+    return (3 if team else 8) // per_cta * per_cta * torch.cuda.get_device_properties(0).multi_processor_count
+
+
+def train(V, walks, counts, **options):
+    opt = sgns.default_options(iter=1, engine="persistent", table_size=1000000, sample=0.0, **options)
+    with sgns.Trainer(opt) as t:
+        t.set_vocab(counts)
+        return t.train_corpus(walks)
+
+
+@pytest.mark.parametrize("V,d,window,negative,storage,workers", [
+    (400_000, 200, 7, 3, "bf16", 0), (1_100_000, 128, 10, 5, "bf16", 0), (190_000, 256, 10, 10, "fp32", 0),
+    (20_000, 128, 10, 5, "fp32", 700), (20_000, 64, 5, 5, "bf16", 5000)])
+def test_tried_shapes_hold_every_worker(V, d, window, negative, storage, workers, sgns_lib, capfd):
+    """The autotuner tries shapes that hold all the workers of the call; when none does, it tries
+    the one-warp shapes."""
+    walks, counts = small_corpus(V, 6000, seed=V)
+    st = train(V, walks, counts, size=d, window=window, negative=negative, storage=storage, workers=workers, debug=3)
+    trials = re.findall(r"trial team (\d), (\d) per CTA.*?: (\d+) workers", capfd.readouterr().err)
+    assert trials and st.workers == (workers or int(trials[0][2]))
+    for team, per_cta, n in trials:
+        assert int(n) == st.workers
+        assert int(n) <= held(int(team), int(per_cta)) or (not int(team) and workers == 5000), (team, per_cta, n)
