@@ -588,13 +588,30 @@ bool teams_allowed(const sgns_options& o) { return o.forward_tile == 0 && !o.com
 // The forward tile reported when none is given.
 int default_tile(const sgns_handle* h) { return h->opt.forward_tile > 0 ? h->opt.forward_tile : 1; }
 
-// The engine of a given CTA shape (sets team and tile): a team per worker where wpc of them
-// fit a CTA, else one warp per worker.
-void shape_for_wpc(sgns_handle* h, int wpc) {
+// Whether the GPU holds n workers (at least one) of a shape at once; the shape becomes the
+// handle's.
+bool holds(sgns_handle* h, const Shape& c, int64_t n) {
+  int64_t resident = 0;
+  h->team = c.team;
+  h->tile = c.tile;
+  h->wpc = c.wpc;
+  return resident_workers(h, c.wpc, &resident) == SGNS_OK && resident >= std::max<int64_t>(n, 1);
+}
+
+// The engine of wpc workers per CTA, untimed: a team per worker where all of them run at once,
+// else one warp per worker.  While all run at once a team is the faster at every size measured
+// (200k vertices, 1 / 2 / 3 workers per SM, team against one warp in ms: d = 64, bf16 17.6 /
+// 10.3 / 8.2 against 37.8 / 19.3 / 13.0; d = 128, bf16 19.0 / 11.4 / 9.3 against 42.4 / 21.6 /
+// 14.6; d = 256, K = 10, fp32 43.9 / 25.1 / 20.3 against 87.0 / 44.4 / 32.2; d = 16 alike).  In
+// two waves it is not (456 workers in CTAs of two, d = 128, bf16: 14.9 against 14.8).
+void shape_for_wpc(sgns_handle* h, int wpc, int workers) {
+  if (teams_allowed(h->opt) && wpc <= kTeamMaxPerCta && holds(h, Shape{true, wpc, 1}, workers)) {
+    h->tile = default_tile(h);
+    return;
+  }
+  h->team = false;
+  h->wpc = wpc;
   h->tile = default_tile(h);
-  int resident = 0;
-  h->team = teams_allowed(h->opt) && wpc <= kTeamMaxPerCta;
-  if (h->team && persistent_shape(h, wpc, &resident) != SGNS_OK) h->team = false;
 }
 
 // Autotuner: times launch shapes of the persistent engine on a prefix of the corpus, on
@@ -616,8 +633,7 @@ sgns_status autotune(sgns_handle* h) {
     h->wpc = c.wpc;
   };
   if (o.warps_per_cta > 0) {  // a given CTA shape
-    h->wpc = o.warps_per_cta;
-    shape_for_wpc(h, h->wpc);
+    shape_for_wpc(h, o.warps_per_cta, o.workers > 0 ? o.workers : rule_workers(h, o.warps_per_cta));
     h->workers = o.workers;
     if (!h->workers) {
       sgns_status st = persistent_shape(h, h->wpc, &h->workers);
@@ -633,13 +649,8 @@ sgns_status autotune(sgns_handle* h) {
   // as many at once as fit.
   const int want = o.workers > 0 ? o.workers : rule;
   std::vector<Shape> shapes;
-  auto holds = [&](const Shape& c, int64_t n) {
-    int64_t resident = 0;
-    use(c);
-    return resident_workers(h, c.wpc, &resident) == SGNS_OK && resident >= std::max<int64_t>(n, 1);
-  };
   auto consider = [&](const Shape& c, int64_t n) {
-    if (holds(c, n)) shapes.push_back(c);
+    if (holds(h, c, n)) shapes.push_back(c);
   };
   if (teams_allowed(o))
     for (int wpc = 1; wpc <= kTeamMaxPerCta; wpc++) consider(Shape{true, wpc, 1}, want);
@@ -650,7 +661,7 @@ sgns_status autotune(sgns_handle* h) {
   if (shapes.empty()) return fail(h, SGNS_EINVAL, "no persistent-engine shape fits this configuration");
   Shape cached{};
   if (tune_cache_lookup(key, &cached) && (!cached.team || teams_allowed(o)) &&
-      holds(cached, all_held || cached.team ? want : 1)) {
+      holds(h, cached, all_held || cached.team ? want : 1)) {
     if (!window_engine_has_tile2(o.size, o.negative)) cached.tile = 1;
     if (o.forward_tile > 0) cached.tile = o.forward_tile;
     use(cached);
@@ -1112,10 +1123,9 @@ sgns_status sgns_train(sgns_handle* h) {
   sgns_status st;
   const bool exact = h->opt.mode == SGNS_MODE_REPLAY_EXACT;
   if (h->opt.engine == SGNS_ENGINE_PERSISTENT) {
-    if (exact) {  // one worker in a one-warp CTA: nothing to tune
+    if (exact) {  // one worker: nothing to tune
       workers = 1;
-      h->wpc = h->opt.warps_per_cta > 0 ? h->opt.warps_per_cta : 1;
-      shape_for_wpc(h, h->wpc);
+      shape_for_wpc(h, h->opt.warps_per_cta > 0 ? h->opt.warps_per_cta : 1, 1);
       st = run_persistent(h, 1, h->wpc, true, &ms);
       if (st) return st;
       return finish_stats(h, workers, ms);

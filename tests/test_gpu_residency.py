@@ -47,3 +47,20 @@ def test_tried_shapes_hold_every_worker(V, d, window, negative, storage, workers
     for team, per_cta, n in trials:
         assert int(n) == st.workers
         assert int(n) <= held(int(team), int(per_cta)) or (not int(team) and workers == 5000), (team, per_cta, n)
+
+
+@pytest.mark.parametrize("per_cta,per_sm,more,warps", [(1, 1, 0, 5), (1, 3, 0, 5), (1, 3, 1, 1), (2, 2, 0, 5), (2, 2, 1, 1),
+                                                       (3, 3, 0, 5), (3, 3, 1, 1), (4, 1, 0, 1)])
+def test_given_cta_shape_takes_teams_where_all_run_at_once(per_cta, per_sm, more, warps, sgns_lib):
+    walks, counts = small_corpus(20_000, 6000, seed=5)
+    workers = held(0, 1) // 8 * per_sm + more
+    st = train(20_000, walks, counts, size=64, window=5, negative=5, storage="bf16", workers=workers,
+               warps_per_cta=per_cta, debug=0)
+    assert (st.workers, st.warps_per_cta, st.warps_per_worker) == (workers, per_cta, warps)
+
+
+def test_given_cta_shape_at_the_default_count(sgns_lib):
+    """400,000 vertices, CTAs of two: a count of its own rule, above the teams that run at once."""
+    walks, counts = small_corpus(400_000, 6000, seed=6)
+    st = train(400_000, walks, counts, size=128, window=10, negative=5, storage="bf16", warps_per_cta=2, debug=0)
+    assert held(1, 1) < st.workers <= held(0, 2) and st.warps_per_worker == 1
