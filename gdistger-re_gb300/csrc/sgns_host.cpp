@@ -625,7 +625,8 @@ void shape_for_wpc(sgns_handle* h, int wpc, int workers) {
 sgns_status autotune(sgns_handle* h) {
   const sgns_options& o = h->opt;
   const std::string key = tune_key(h);
-  int rule = 0;  // the default worker count: the most that any CTA shape's rule gives
+  int rule = 0;  // the default worker count: the most that any CTA shape's rule gives (a worker
+                 // takes at most 97 KB of an SM's 228: never 0)
   for (int wpc = 1; wpc <= 8; wpc++) rule = std::max(rule, rule_workers(h, wpc));
   auto use = [&](const Shape& c) {
     h->team = c.team;
@@ -697,23 +698,27 @@ sgns_status autotune(sgns_handle* h) {
   sgns_status st = SGNS_OK;
   cudaError_t e;
   if ((e = cudaMalloc(&wih_s, tbytes)) != cudaSuccess || (e = cudaMalloc(&woh_s, tbytes)) != cudaSuccess) {
-    // no room for scratch tables: untimed, the one-warp shape with the most workers (a warp
-    // each fills the GPU best), or what fits
+    // no room for scratch tables: untimed, the first shape that holds all the workers (teams
+    // before one warp per worker, as in shape_for_wpc; small CTAs spread best), or the one
+    // that holds most of them
     restore();
     cudaGetLastError();
+    int64_t best_held = 0;
     for (const Shape& c : shapes) {
-      int workers = 0;
+      int64_t resident = 0;
       use(c);
-      if (persistent_shape(h, c.wpc, &workers) == SGNS_OK && (workers > best_workers || (best_shape.team && !c.team))) {
+      if (resident_workers(h, c.wpc, &resident) != SGNS_OK) continue;
+      if (std::min<int64_t>(resident, want) > best_held) {
         best_shape = c;
-        best_workers = workers;
+        best_held = std::min<int64_t>(resident, want);
       }
     }
     use(best_shape);
-    h->workers = o.workers > 0 ? o.workers : rule > 0 ? rule : best_workers;
+    h->workers = want;
     h->tuned = true;
     if (o.debug > 0)
-      fprintf(stderr, "sgns: no memory for autotuning; persistent engine at %d warps/CTA\n", best_shape.wpc);
+      fprintf(stderr, "sgns: no memory for autotuning; persistent engine: team %d, %d workers/CTA\n", (int)best_shape.team,
+              best_shape.wpc);
     return SGNS_OK;
   }
   if ((e = cudaMemcpyAsync(wih_s, h->wih, tbytes, cudaMemcpyDeviceToDevice, h->stream)) != cudaSuccess ||

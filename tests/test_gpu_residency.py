@@ -64,3 +64,25 @@ def test_given_cta_shape_at_the_default_count(sgns_lib):
     walks, counts = small_corpus(400_000, 6000, seed=6)
     st = train(400_000, walks, counts, size=128, window=10, negative=5, storage="bf16", warps_per_cta=2, debug=0)
     assert held(1, 1) < st.workers <= held(0, 2) and st.warps_per_worker == 1
+
+
+def test_untimed_shape_is_the_faster_engine(sgns_lib):
+    """No room for the autotuner's copies of the tables: teams where the GPU holds all of them
+    (here 450 workers), which the timings prefer at every count of theirs."""
+    import torch
+
+    from test_gpu_parity import _hold_all_but
+
+    V = 180_000
+    walks, counts = small_corpus(V, 6000, seed=7)
+    opt = sgns.default_options(size=256, window=5, negative=5, iter=1, debug=0, table_size=1000000, sample=0.0)
+    with sgns.Trainer(opt) as t:
+        t.set_vocab(counts)  # two tables of 184 MB
+        t.upload(walks)
+        hold = _hold_all_but(276 << 20)
+        try:
+            st = t.train()
+        finally:
+            del hold
+            torch.cuda.empty_cache()
+    assert st.workers == V // 400 and st.warps_per_worker == 5
