@@ -525,18 +525,26 @@ sgns_status run_plain(sgns_handle* h, int workers, float* ms_out) {
   return SGNS_OK;
 }
 
-// Autotuner: times each CTA shape of the persistent engine on a prefix of the corpus,
-// on scratch copies of the tables, and keeps the fastest (pairs per second).
-// Autotuner cache: with SGNS_TUNE_CACHE naming a file, the chosen CTA shape is kept per
-// device model and problem shape ("key<TAB>warps_per_cta" lines) and reused by later runs.
-// The file is only an optimisation: any error reading or writing it is ignored.
+// Teams train the workers unless the options ask for what only the one-warp kernel does: a
+// forward tile, the loss, one walk per step.
+bool teams_allowed(const sgns_options& o) { return o.forward_tile == 0 && !o.compute_loss && o.windows_per_step != 1; }
+
+// Autotuner cache: with SGNS_TUNE_CACHE naming a file, the chosen launch shape is kept per
+// device model and problem shape and reused by later runs.  The file is only an
+// optimisation: any error reading or writing it is ignored.  The key holds what the choice
+// depends on: the sizes (V because the default worker count is capped at V/400), which shapes
+// the options leave to choose from and which kernel they time, and the generation of the
+// kernels, which goes up when their order may have changed (lines of other generations are
+// not taken; those of the first end with V).
+constexpr int kTuneGeneration = 2;
 std::string tune_key(const sgns_handle* h) {
   cudaDeviceProp prop{};
   if (cudaGetDeviceProperties(&prop, h->opt.device) != cudaSuccess) prop.name[0] = 0;
   char key[384];
-  // V enters the key because the default worker count is capped at V/400
-  snprintf(key, sizeof key, "%s|sms=%d|d=%d|w=%d|K=%d|storage=%d|lmax=%d|workers=%d|V=%lld", prop.name, h->num_sms,
-           h->opt.size, h->opt.window, h->opt.negative, h->opt.storage, h->lmax, h->opt.workers, (long long)h->V);
+  const sgns_options& o = h->opt;
+  snprintf(key, sizeof key, "%s|sms=%d|d=%d|w=%d|K=%d|storage=%d|lmax=%d|workers=%d|V=%lld|teams=%d|loss=%d|windows=%d|gen=%d",
+           prop.name, h->num_sms, o.size, o.window, o.negative, o.storage, h->lmax, o.workers, (long long)h->V,
+           (int)teams_allowed(o), (int)(o.compute_loss != 0), o.windows_per_step == 1 ? 1 : 2, kTuneGeneration);
   for (char* c = key; *c; c++)
     if (*c == '\t' || *c == '\n') *c = ' ';
   return key;
@@ -581,10 +589,6 @@ void tune_cache_store(const std::string& key, const Shape& c) {
   }
 }
 
-// Teams train the workers unless the options ask for what only the one-warp kernel does: a
-// forward tile, the loss, one walk per step.
-bool teams_allowed(const sgns_options& o) { return o.forward_tile == 0 && !o.compute_loss && o.windows_per_step != 1; }
-
 // The forward tile reported when none is given.
 int default_tile(const sgns_handle* h) { return h->opt.forward_tile > 0 ? h->opt.forward_tile : 1; }
 
@@ -619,9 +623,6 @@ void shape_for_wpc(sgns_handle* h, int wpc, int workers) {
 // train the workers and an SM holds as many as it gets: a team per worker at 1, 2 and 3 workers
 // per CTA (few workers spread best in small CTAs) and one warp per worker at 4..8 (the shapes
 // that fill an SM); else one warp per worker at 1..8.
-// Autotuner cache: with SGNS_TUNE_CACHE naming a file, the choice is kept per device model
-// and problem shape and reused by later runs.  The file is only an optimisation: any error
-// reading or writing it is ignored.
 sgns_status autotune(sgns_handle* h) {
   const sgns_options& o = h->opt;
   const std::string key = tune_key(h);
