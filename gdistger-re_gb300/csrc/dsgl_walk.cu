@@ -461,23 +461,17 @@ static int walk_block_threads(int max_length) {
 
 size_t walk_scratch_bytes(int64_t walker_num) {
   const int64_t tiles = (walker_num + kScanBlock - 1) / kScanBlock;
-  return sizeof(int32_t) * (size_t)walker_num + sizeof(int64_t) * (size_t)(walker_num + 1) +
-         sizeof(int64_t) * (size_t)(tiles + 1) + 64;
+  return sizeof(int32_t) * (size_t)walker_num + sizeof(int64_t) * (size_t)(tiles + 1);
 }
 
-// Pass 1 (lengths) and the scan; *offsets_out points into scratch (walker_num + 1 entries,
-// the last = total tokens).
+// Pass 1 (lengths) and the scan: offsets, walker_num + 1 entries, the last = total tokens.
 cudaError_t launch_info_walks_count(const int64_t* indptr, const int32_t* indices, const int32_t* cn,
                                     const double* xl, const double* len_table, int64_t V, int64_t walker_num,
                                     int min_length, int max_length, double r_threshold, uint64_t seed, int trace,
-                                    void* scratch, int num_sms, int64_t** offsets_out, cudaStream_t s) {
-  char* p = static_cast<char*>(scratch);
-  int64_t* offsets = reinterpret_cast<int64_t*>(p);
-  p += sizeof(int64_t) * (size_t)(walker_num + 1);
+                                    void* scratch, int num_sms, int64_t* offsets, cudaStream_t s) {
   const int64_t tiles = (walker_num + kScanBlock - 1) / kScanBlock;
-  int64_t* tile_sums = reinterpret_cast<int64_t*>(p);
-  p += sizeof(int64_t) * (size_t)(tiles + 1);
-  int32_t* lengths = reinterpret_cast<int32_t*>(p);
+  int64_t* tile_sums = static_cast<int64_t*>(scratch);
+  int32_t* lengths = reinterpret_cast<int32_t*>(tile_sums + tiles + 1);
   const WalkArgs a{indptr, indices, cn, xl, reinterpret_cast<const LengthTable*>(len_table), V, walker_num, min_length,
                    max_length, r_threshold, seed, trace, lengths, nullptr, nullptr};
   const int T = walk_block_threads(max_length);
@@ -494,7 +488,6 @@ cudaError_t launch_info_walks_count(const int64_t* indptr, const int32_t* indice
   scan_tiles_kernel<<<(unsigned)tiles, kScanBlock, 0, s>>>(lengths, walker_num, offsets, tile_sums);
   scan_tile_sums_kernel<<<1, kScanBlock, 0, s>>>(tile_sums, tiles);
   add_tile_offsets_kernel<<<(unsigned)((walker_num + 256) / 256), 256, 0, s>>>(offsets, walker_num, tile_sums, tiles);
-  *offsets_out = offsets;
   return cudaGetLastError();
 }
 

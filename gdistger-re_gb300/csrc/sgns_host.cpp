@@ -1616,60 +1616,139 @@ sgns_status sgns_edge_common_neighbors(const int64_t* indptr, const int32_t* ind
   return SGNS_OK;
 }
 
-sgns_status sgns_info_walks(const sgns_walk_options* o, const int64_t* indptr, const int32_t* indices,
-                            const int32_t* cn, int64_t V, int64_t n_edges, int32_t* corpus, int64_t cap,
-                            int64_t* n_tokens, void* stream) {
-  NvtxRange r_("sgns_info_walks");
-  if (!o || !n_tokens || V < 1 || V > INT32_MAX || n_edges < 0 || !indptr || (n_edges > 0 && (!indices || !cn)) ||
-      cap < 0 || (cap > 0 && !corpus))
-    return fail(nullptr, SGNS_EINVAL, "bad walk arguments");
+namespace {
+sgns_status check_walk_options(const sgns_walk_options* o) {
   if (o->walker_num < 0 || o->min_length < 0 || o->max_length < 1 || o->max_length > kWalkMaxLength ||
       !(o->r_threshold == o->r_threshold) || (o->trace_steps != 0 && o->trace_steps != 1))
     return fail(nullptr, SGNS_EINVAL,
                 "walk options: walker_num >= 0, min_length >= 0, max_length in [1, %d], trace_steps 0 or 1",
                 kWalkMaxLength);
+  return SGNS_OK;
+}
+
+// A walk call's graph, stream and device, and the device's scratch (locked while it lives).
+struct WalkCall {
+  const sgns_walk_options* o;
+  const int64_t* indptr;
+  const int32_t *indices, *cn;
+  int64_t V, n_edges;
+  cudaStream_t s;
+  int sms;
+  DeviceScratch* ds;
+  std::unique_lock<std::mutex> lock;
+
+  sgns_status open() {
+    sms = device_sms();
+    ds = sms ? device_scratch() : nullptr;
+    if (!ds) return fail(nullptr, SGNS_ECUDA, "no current CUDA device");
+    lock = std::unique_lock<std::mutex>(ds->mx);
+    return SGNS_OK;
+  }
+  // Scratch: a status word, x log2 x, the per-length constants of the update, the length
+  // pass's own, then (own_offsets) the offsets where the caller brings none.
+  static constexpr int kEntries = kWalkMaxLength + 2;
+  static constexpr size_t kTables = sizeof(double) * (size_t)kEntries * (1 + kWalkTableDoubles);
+  size_t offsets_at() const { return (256 + kTables + walk_scratch_bytes(o->walker_num) + 7) & ~(size_t)7; }
+  size_t bytes(bool own_offsets) const {
+    return offsets_at() + (own_offsets ? sizeof(int64_t) * (size_t)(o->walker_num + 1) : 0);
+  }
+  char* at(size_t off) const { return static_cast<char*>(ds->buf) + off; }
+
+  // the walks' lengths, scanned into offsets (null: the scratch's own)
+  sgns_status count(int64_t*& offsets, int64_t* total) {
+    sgns_status st = ds->ensure(bytes(!offsets));
+    if (st) return st;
+    if (!offsets) offsets = reinterpret_cast<int64_t*>(at(offsets_at()));
+    double* xl = reinterpret_cast<double*>(at(256));
+    if ((st = check_csr("walks", indptr, indices, V, n_edges, reinterpret_cast<int32_t*>(at(0)), sms, s))) return st;
+    std::vector<double> tables(kTables / sizeof(double));
+    xlog2x_table(kEntries, tables.data());
+    walk_length_table(kEntries, tables.data(), tables.data() + kEntries);
+    cudaError_t e;
+    if ((e = cudaMemcpyAsync(xl, tables.data(), kTables, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
+        (e = launch_info_walks_count(indptr, indices, cn, xl, xl + kEntries, V, o->walker_num, o->min_length,
+                                     o->max_length, o->r_threshold, o->seed, o->trace_steps, at(256 + kTables), sms,
+                                     offsets, s)) != cudaSuccess)
+      return fail(nullptr, SGNS_ECUDA, "walks: %s", cudaGetErrorString(e));
+    return read_total(offsets, total);
+  }
+  sgns_status read_total(const int64_t* offsets, int64_t* total) {
+    cudaError_t e;
+    if ((e = cudaMemcpyAsync(total, offsets + o->walker_num, sizeof *total, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(s)) != cudaSuccess)
+      return fail(nullptr, SGNS_ECUDA, "walks: %s", cudaGetErrorString(e));
+    return SGNS_OK;
+  }
+  sgns_status emit(const int64_t* offsets, int32_t* corpus) {
+    cudaError_t e;
+    if ((e = launch_info_walks_emit(indptr, indices, cn, V, o->walker_num, o->seed, o->trace_steps, offsets, corpus,
+                                    sms, s)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(s)) != cudaSuccess)
+      return fail(nullptr, SGNS_ECUDA, "walks: %s", cudaGetErrorString(e));
+    return SGNS_OK;
+  }
+};
+
+bool bad_walk_graph(const int64_t* indptr, const int32_t* indices, const int32_t* cn, int64_t V, int64_t n_edges) {
+  return V < 1 || V > INT32_MAX || n_edges < 0 || !indptr || (n_edges > 0 && (!indices || !cn));
+}
+}  // namespace
+
+sgns_status sgns_info_walks(const sgns_walk_options* o, const int64_t* indptr, const int32_t* indices,
+                            const int32_t* cn, int64_t V, int64_t n_edges, int32_t* corpus, int64_t cap,
+                            int64_t* n_tokens, void* stream) {
+  NvtxRange r_("sgns_info_walks");
+  if (!o || !n_tokens || bad_walk_graph(indptr, indices, cn, V, n_edges) || cap < 0 || (cap > 0 && !corpus))
+    return fail(nullptr, SGNS_EINVAL, "bad walk arguments");
+  sgns_status st = check_walk_options(o);
+  if (st) return st;
   *n_tokens = 0;
   if (o->walker_num == 0) return SGNS_OK;
-  const int sms = device_sms();
-  if (!sms) return fail(nullptr, SGNS_ECUDA, "no current CUDA device");
-  DeviceScratch* ds = device_scratch();
-  if (!ds) return fail(nullptr, SGNS_ECUDA, "no current CUDA device");
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  std::lock_guard<std::mutex> g(ds->mx);
-  // x log2 x, then the per-length constants of the update
-  constexpr int kEntries = kWalkMaxLength + 2;
-  const size_t xl_bytes = sizeof(double) * (size_t)kEntries, tab_bytes = xl_bytes * (1 + kWalkTableDoubles);
-  sgns_status st = ds->ensure(256 + tab_bytes + walk_scratch_bytes(o->walker_num));
-  if (st) return st;
-  char* base = static_cast<char*>(ds->buf);
-  int32_t* status = reinterpret_cast<int32_t*>(base);
-  double* xl = reinterpret_cast<double*>(base + 256);
-  void* scratch = base + 256 + tab_bytes;
-  if ((st = check_csr("walks", indptr, indices, V, n_edges, status, sms, s))) return st;
-  std::vector<double> tables(tab_bytes / sizeof(double));
-  xlog2x_table(kEntries, tables.data());
-  walk_length_table(kEntries, tables.data(), tables.data() + kEntries);
+  WalkCall c{o, indptr, indices, cn, V, n_edges, static_cast<cudaStream_t>(stream), 0, nullptr, {}};
   int64_t* offsets = nullptr;
   int64_t total = 0;
-  cudaError_t e;
-  if ((e = cudaMemcpyAsync(xl, tables.data(), tab_bytes, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
-      (e = launch_info_walks_count(indptr, indices, cn, xl, xl + kEntries, V, o->walker_num, o->min_length,
-                                   o->max_length, o->r_threshold, o->seed, o->trace_steps, scratch, sms, &offsets,
-                                   s)) != cudaSuccess ||
-      (e = cudaMemcpyAsync(&total, offsets + o->walker_num, sizeof total, cudaMemcpyDeviceToHost, s)) !=
-          cudaSuccess ||
-      (e = cudaStreamSynchronize(s)) != cudaSuccess)
-    return fail(nullptr, SGNS_ECUDA, "walks: %s", cudaGetErrorString(e));
+  if ((st = c.open()) || (st = c.count(offsets, &total))) return st;
   *n_tokens = total;
   if (total > cap) {
     if (cap == 0 && !corpus) return SGNS_OK;
     return fail(nullptr, SGNS_EINVAL, "walks yield %lld tokens, capacity %lld", (long long)total, (long long)cap);
   }
-  if ((e = launch_info_walks_emit(indptr, indices, cn, V, o->walker_num, o->seed, o->trace_steps, offsets, corpus, sms,
-                                  s)) != cudaSuccess ||
-      (e = cudaStreamSynchronize(s)) != cudaSuccess)
-    return fail(nullptr, SGNS_ECUDA, "walks: %s", cudaGetErrorString(e));
-  return SGNS_OK;
+  return c.emit(offsets, corpus);
+}
+
+sgns_status sgns_info_walk_offsets(const sgns_walk_options* o, const int64_t* indptr, const int32_t* indices,
+                                   const int32_t* cn, int64_t V, int64_t n_edges, int64_t* offsets, int64_t* n_tokens,
+                                   void* stream) {
+  NvtxRange r_("sgns_info_walk_offsets");
+  if (!o || !n_tokens || bad_walk_graph(indptr, indices, cn, V, n_edges) || !offsets)
+    return fail(nullptr, SGNS_EINVAL, "bad walk arguments");
+  sgns_status st = check_walk_options(o);
+  if (st) return st;
+  *n_tokens = 0;
+  if (o->walker_num == 0) return SGNS_OK;
+  WalkCall c{o, indptr, indices, cn, V, n_edges, static_cast<cudaStream_t>(stream), 0, nullptr, {}};
+  if ((st = c.open())) return st;
+  return c.count(offsets, n_tokens);
+}
+
+sgns_status sgns_info_walk_tokens(const sgns_walk_options* o, const int64_t* indptr, const int32_t* indices,
+                                  const int32_t* cn, int64_t V, int64_t n_edges, const int64_t* offsets,
+                                  int32_t* corpus, int64_t cap, void* stream) {
+  NvtxRange r_("sgns_info_walk_tokens");
+  if (!o || bad_walk_graph(indptr, indices, cn, V, n_edges) || !offsets || cap < 0 || (cap > 0 && !corpus))
+    return fail(nullptr, SGNS_EINVAL, "bad walk arguments");
+  sgns_status st = check_walk_options(o);
+  if (st) return st;
+  if (o->walker_num == 0) return SGNS_OK;
+  WalkCall c{o, indptr, indices, cn, V, n_edges, static_cast<cudaStream_t>(stream), 0, nullptr, {}};
+  int64_t total = 0;
+  if ((st = c.open()) || (st = c.ds->ensure(64)) ||
+      (st = check_csr("walks", indptr, indices, V, n_edges, reinterpret_cast<int32_t*>(c.at(0)), c.sms, c.s)) ||
+      (st = c.read_total(offsets, &total)))
+    return st;
+  if (total < 0 || total > cap)
+    return fail(nullptr, SGNS_EINVAL, "walks yield %lld tokens, capacity %lld", (long long)total, (long long)cap);
+  return c.emit(offsets, corpus);
 }
 
 sgns_status sgns_loss_adjoint(int32_t dtype, int32_t d, int64_t V, int32_t n, const int32_t* in_ptr,

@@ -242,7 +242,7 @@ constexpr int kWalkTableDoubles = 4;
 cudaError_t launch_info_walks_count(const int64_t* indptr, const int32_t* indices, const int32_t* cn,
                                     const double* xl, const double* len_table, int64_t V, int64_t walker_num,
                                     int min_length, int max_length, double r_threshold, uint64_t seed, int trace,
-                                    void* scratch, int num_sms, int64_t** offsets_out, cudaStream_t s);
+                                    void* scratch, int num_sms, int64_t* offsets, cudaStream_t s);
 cudaError_t launch_info_walks_emit(const int64_t* indptr, const int32_t* indices, const int32_t* cn, int64_t V,
                                    int64_t walker_num, uint64_t seed, int trace, const int64_t* offsets,
                                    int32_t* corpus, int num_sms, cudaStream_t s);

@@ -106,6 +106,9 @@ def lib():
         L.sgns_edge_common_neighbors.argtypes = [vp, vp, i64, i64, vp, vp]
         L.sgns_info_walks.argtypes = [ctypes.POINTER(WalkOptions), vp, vp, vp, i64, i64, vp, i64,
                                       ctypes.POINTER(i64), vp]
+        L.sgns_info_walk_offsets.argtypes = [ctypes.POINTER(WalkOptions), vp, vp, vp, i64, i64, vp,
+                                             ctypes.POINTER(i64), vp]
+        L.sgns_info_walk_tokens.argtypes = [ctypes.POINTER(WalkOptions), vp, vp, vp, i64, i64, vp, vp, i64, vp]
         L.sgns_internal_host_vocab.argtypes = [vp, i64, ctypes.c_float, i64, i32, vp, vp, vp, vp,
                                                ctypes.POINTER(ctypes.c_uint64)]
         L.sgns_internal_host_vocab.restype = i32
@@ -367,14 +370,10 @@ def edge_common_neighbors(indptr, indices, cn, stream=0):
                                             cn.data_ptr() if E else None, ctypes.c_void_p(stream)))
 
 
-# Bytes that info_walks takes for a moment to make a corpus of unknown size in one call.
-_WALK_ROOM = 4 << 30
-
-
 def info_walks(indptr, indices, cn, walker_num, min_length=20, max_length=80, r_threshold=0.999, seed=1,
                corpus=None, stream=0, trace=1):
     """sgns_info_walks on device tensors.  corpus: int32 device tensor to fill (None: a new
-    one of the exact size).  Returns (corpus, n_tokens)."""
+    one of the exact size, between the lengths and the tokens).  Returns (corpus, n_tokens)."""
     import torch
 
     V, E = int(indptr.numel()) - 1, int(indices.numel())
@@ -382,16 +381,18 @@ def info_walks(indptr, indices, cn, walker_num, min_length=20, max_length=80, r_
                     r_threshold=float(r_threshold), seed=int(seed), trace_steps=int(trace))
     n = ctypes.c_int64()
     args = (indptr.data_ptr(), indices.data_ptr() if E else None, cn.data_ptr() if E else None, V, E)
-    most = o.walker_num * (o.max_length + 1)
-    if corpus is None and 0 < 4 * most <= _WALK_ROOM:  # one call into room for the longest walks
+    if corpus is None:  # the lengths, then a corpus of their sum
         try:
-            room = torch.empty(most, dtype=torch.int32, device=indptr.device)
-        except torch.cuda.OutOfMemoryError:
-            room = None
-        if room is not None:
-            _check(lib().sgns_info_walks(ctypes.byref(o), *args, room.data_ptr(), most, ctypes.byref(n),
-                                         ctypes.c_void_p(stream)))
-            return room[:n.value].clone(), n.value
+            offsets = torch.empty(max(o.walker_num, 0) + 1, dtype=torch.int64, device=indptr.device)
+        except RuntimeError:  # no room for 8 bytes a walk
+            offsets = None
+        if offsets is not None:
+            _check(lib().sgns_info_walk_offsets(ctypes.byref(o), *args, offsets.data_ptr(), ctypes.byref(n),
+                                                ctypes.c_void_p(stream)))
+            corpus = torch.empty(max(n.value, 1), dtype=torch.int32, device=indptr.device)
+            _check(lib().sgns_info_walk_tokens(ctypes.byref(o), *args, offsets.data_ptr(), corpus.data_ptr(), n.value,
+                                               ctypes.c_void_p(stream)))
+            return corpus[:n.value], n.value
     if corpus is None:  # a counting call first: the length pass runs twice
         _check(lib().sgns_info_walks(ctypes.byref(o), *args, None, 0, ctypes.byref(n), ctypes.c_void_p(stream)))
         corpus = torch.empty(max(n.value, 1), dtype=torch.int32, device=indptr.device)

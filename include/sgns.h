@@ -299,6 +299,18 @@ sgns_status sgns_info_walks(const sgns_walk_options* opt, const int64_t* indptr,
                             const int32_t* cn, int64_t V, int64_t n_edges, int32_t* corpus, int64_t cap,
                             int64_t* n_tokens, void* stream);
 
+/* The same in two calls, for a corpus of unknown size: the pass over the walks' lengths runs
+ * once and the corpus is allocated in between.  offsets: device memory, walker_num + 1
+ * entries: walk k's first token and, last, *n_tokens (nothing is written for no walkers).
+ * The second call takes the offsets as the first one wrote them for the same options and
+ * graph; cap below the last of them: SGNS_EINVAL and nothing written. */
+sgns_status sgns_info_walk_offsets(const sgns_walk_options* opt, const int64_t* indptr, const int32_t* indices,
+                                   const int32_t* cn, int64_t V, int64_t n_edges, int64_t* offsets,
+                                   int64_t* n_tokens, void* stream);
+sgns_status sgns_info_walk_tokens(const sgns_walk_options* opt, const int64_t* indptr, const int32_t* indices,
+                                  const int32_t* cn, int64_t V, int64_t n_edges, const int64_t* offsets,
+                                  int32_t* corpus, int64_t cap, void* stream);
+
 /* SGNS loss and its hand-written adjoint for n minibatches that index tables of V
  * rows (device pointers).  Minibatch b has inputs in_ids[in_ptr[b]..in_ptr[b+1]), the
  * first in_first[b] of them labelled by output 0 and the rest by the last output, and

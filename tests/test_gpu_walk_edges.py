@@ -54,3 +54,52 @@ def test_walks_at_the_edges(min_length, max_length, r_th, trace, sgns_lib, oracl
     got, n = sgns.info_walks(dip, dix, torch.from_numpy(cn).cuda(), 777, min_length, max_length, r_th, 11, trace=trace)
     want, _ = oracle_mod.info_walks(ip, ix, cn, 777, min_length, max_length, r_th, 11, trace=trace)
     assert n == len(want) and np.array_equal(got.cpu().numpy(), want)
+
+
+def test_walks_without_a_corpus_take_its_room_only(sgns_lib):
+    """A new corpus costs its own bytes and the walks' offsets, not those of the longest walks
+    (here 800 MB for about 20): what torch keeps, the library cannot allocate."""
+    import torch
+
+    V, n_walks = 4000, 200_000
+    ip = torch.arange(0, 2 * V + 1, 2, dtype=torch.int64, device="cuda")
+    i = torch.arange(V, dtype=torch.int32, device="cuda")
+    ix = torch.stack([(i + V - 1) % V, (i + 1) % V], 1).sort(1).values.reshape(-1).contiguous()
+    cn = torch.zeros(2 * V, dtype=torch.int32, device="cuda")
+    torch.cuda.empty_cache()
+    torch.cuda.reset_peak_memory_stats()
+
+    def asked():  # bytes asked for, without the allocator's rounding
+        return torch.cuda.memory_stats()["requested_bytes.all.peak"]
+
+    before, reserved = asked(), torch.cuda.memory_reserved()
+    out, n = sgns.info_walks(ip, ix, cn, n_walks, 20, 1000, 0.999, 3, trace=0)
+    peak, kept = asked() - before, torch.cuda.max_memory_reserved() - reserved
+    room = 4 * n + 8 * (n_walks + 1) + (1 << 16)
+    assert n == out.numel() and 8 * room < 4 * 1001 * n_walks
+    assert peak <= room and kept <= 2 * room + (64 << 20)
+    assert int((out == -1).sum()) == n_walks
+
+
+def test_walk_tokens_refuse_a_small_corpus(sgns_lib, oracle_mod):
+    """The two calls by themselves: offsets as the corpus's walks, a corpus one entry short
+    refused and left as it was."""
+    import ctypes
+
+    import torch
+
+    ip, ix = clique_and_tail(9, 40)
+    cn = oracle_mod.edge_common_neighbors(ip, ix)
+    want, _ = oracle_mod.info_walks(ip, ix, cn, 500, 5, 40, 0.9, 11, trace=1)
+    dip, dix, dcn = *on_gpu(ip, ix), torch.from_numpy(cn).cuda()
+    o = sgns.WalkOptions(walker_num=500, min_length=5, max_length=40, r_threshold=0.9, seed=11, trace_steps=1)
+    graph = (ctypes.byref(o), dip.data_ptr(), dix.data_ptr(), dcn.data_ptr(), len(ip) - 1, len(ix))
+    offsets, n = torch.empty(501, dtype=torch.int64, device="cuda"), ctypes.c_int64()
+    assert sgns_lib.sgns_info_walk_offsets(*graph, offsets.data_ptr(), ctypes.byref(n), None) == sgns.OK
+    ends = np.flatnonzero(want == -1) + 1
+    assert n.value == len(want) and np.array_equal(offsets.cpu().numpy(), np.append(0, ends))
+    corpus = torch.full((len(want),), -9, dtype=torch.int32, device="cuda")
+    tokens = lambda cap: sgns_lib.sgns_info_walk_tokens(*graph, offsets.data_ptr(), corpus.data_ptr(), cap, None)
+    assert tokens(len(want) - 1) == sgns.EINVAL and bool((corpus == -9).all())
+    assert tokens(len(want)) == sgns.OK and np.array_equal(corpus.cpu().numpy(), want)
+    assert sgns_lib.sgns_info_walk_offsets(*graph, None, ctypes.byref(n), None) == sgns.EINVAL
