@@ -64,8 +64,6 @@ __host__ __device__ __forceinline__ Span span_combine(Span a, Span b) {
 
 __device__ __forceinline__ Span span_identity() { return Span{0ull, 0u, SIG_NONE}; }
 
-__device__ __forceinline__ bool is_digit(uint8_t c) { return c >= '0' && c <= '9'; }
-
 // byte i of the text with a virtual newline at n and blanks after it
 __device__ __forceinline__ uint8_t text_byte(const uint8_t* b, int64_t n, int64_t i) {
   return i < n ? __ldg(b + i) : (i == n ? (uint8_t)'\n' : (uint8_t)' ');

@@ -451,8 +451,8 @@ sgns_status run_persistent(sgns_handle* h, int workers, int wpc, bool use_graph,
   TrainParams p = make_params(h, workers);
   if (use_graph) {
     char key[256];
-    snprintf(key, sizeof key, "%p/%lld/%d/%d/%p/%p/%d/%d/%d/%d", (void*)h->d_corpus, (long long)h->n_tokens,
-             workers, wpc, h->wih, h->woh, h->lmax, h->opt.iter, h->tile, (int)h->team);
+    snprintf(key, sizeof key, "%p/%lld/%d/%d/%p/%p/%d/%d/%d", (void*)h->d_corpus, (long long)h->n_tokens, workers,
+             wpc, h->wih, h->woh, h->lmax, h->opt.iter, (int)h->team);
     if (!h->graph || h->graph_key != key) {
       if (h->graph) cudaGraphExecDestroy(h->graph);
       h->graph = nullptr;
@@ -550,7 +550,7 @@ std::string tune_key(const sgns_handle* h) {
   return key;
 }
 // One launch shape of the persistent engine: a team of warps or one warp per worker, workers
-// per CTA, and the forward tile reported with the one-warp kernel.
+// per CTA, and the forward tile that the statistics report (it selects no kernel).
 struct Shape {
   bool team;
   int wpc, tile;
