@@ -31,8 +31,8 @@
 //     128-column chunk) and leave with one 16-byte atomic add per lane (red.global.add of
 //     four floats; fp64 adds element by element);
 //   * the loss is reduced per warp into 256 fp64 sums;
-//   * sizes and ids are checked on the device (status bits), so a call makes no host round
-//     trip before its launches.
+//   * sizes and ids are checked on the device (status bits); a call reads them back once,
+//     with the sizes that the gradient kernel is launched for.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -477,13 +477,14 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) adjoint_kernel(
 // the output rows widened into shared memory and every gradient an atomic; 845 us with 16
 // warps, the rows read from the ring and sole references stored.  Of a call's 1,048 us (1,550
 // before) the marks take 82, the slots and ids 29, the zeroed rows 46.  What bounds the kernel:
-// issue (57% of cycles, 2,670 warp instructions per minibatch), then its dependent chains.  The next minibatch's ids are
-// loaded at the top of an iteration, its gradient slots with its copies, and the extents
-// one minibatch further ahead.  Rows stay in their storage format in the ring (row stride
-// = row bytes + 16, so lanes reading different rows at one column hit different banks);
-// the output rows are widened once into an fp32 (fp64) copy for the forward's broadcast
-// reads.  Sums keep the order of adjoint_kernel except the forward's dot products, which
-// run as an even and an odd partial sum for fp32.
+// issue (57% of cycles, 2,670 warp instructions per minibatch), then its dependent chains.
+// The next minibatch's ids are loaded at the top of an iteration, its gradient slots with its
+// copies, and the extents one minibatch further ahead.  Rows stay in their storage format in
+// the ring (row stride = row bytes + 16, so lanes reading different rows at one column hit
+// different banks); fp32 and fp64 output rows are also copied once, zero past O, for the
+// forward's broadcast reads; bf16 ones are read from the ring.  Sums keep the order of
+// adjoint_kernel except the forward's dot products, which run as an even and an odd partial
+// sum for fp32, and for bf16 on the tensor cores (forward_mma_bf16).
 
 template <int DT> struct Pipe;
 template <> struct Pipe<0> {  // fp32 rows: 4 elements per 16 bytes

@@ -27,13 +27,15 @@
 // (U) outputMd done, input rows may change; and (B), with the planner: gradients complete,
 // next descriptor written.
 //
-// Measured (GB300, one training pass, against one warp per worker before and now): 100k
-// vertices, 250 workers, d = 128, bf16: 112.5 ms -> 53.6 (one warp: 99); 120k vertices, 300
-// workers, d = 256, K = 10, fp32: 52.7 -> 14.4; one replayed worker, d = 100: 50.9 -> 23.3.
-// A step of a worker alone on its SM takes 6,900 cycles: the forward 1,700, outputMd and the
-// stores 1,900, the updates 800, the planner's arrival another 700.  From about six workers
-// per SM the SM's issue slots are full either way and one warp per worker, which repeats
-// nothing, is faster (1064 workers: 159.7 ms against 211 here); the autotuner measures both.
+// Measured (GB300, kernel time of one training pass, against one warp per worker before and
+// now): 100k vertices, 250 workers, d = 128, bf16: 112.5 ms -> 52.4 (one warp: 98.2); 120k
+// vertices, 300 workers, d = 256, K = 10, fp32: 52.7 -> 14.3 (25.4); one replayed worker, d =
+// 100: 50.9 -> 21.6 (41.2).  A step of a worker alone on its SM takes 6,100 cycles (d = 128,
+// w = 10, bf16), of two 7,150, of three 10,100; with the clock read between its parts (7,050
+// alone) the forward takes 1,930 of them, outputMd and the stores 2,140, the updates 820, the
+// wait for the planner 690, window moves and the other barriers the rest.  160 threads of 128
+// registers: an SM holds three teams, and while it gets no more workers a team is the faster
+// (timings at shape_for_wpc in sgns_host.cpp); beyond, some would wait for others to end.
 //
 // Every sum has the operands and the order of window_engine_kernel (eight partial sums per
 // dot product when d % 16 == 0, else two; outputMd sequential over the inputs; an input's
@@ -161,7 +163,7 @@ __device__ __forceinline__ void plan_worker(const TrainParams& p, const SmallJum
       const unsigned fr = __ballot_sync(kFull, lane < NS && my_r == 0);
       s = __ffs(fr) - 1;
       fresh = true;
-      if (s < 0) {  // cannot happen: at most 2w+2 distinct vertices are resident
+      if (s < 0) {  // cannot happen: a first window holds at most w + 1 rows
         if (lane == 0) atomicExch(&p.ctr->status, 2);
         s = 0;
       }
@@ -619,6 +621,8 @@ __host__ __device__ constexpr int pow2_at_least(int n) {
 
 // S: storage.  OM: output capacity (K + 2 <= OM).  DFIX: d at compile time (0: p.d).  NC:
 // column pairs per lane (half a row holds at most 64 NC columns).
+// One bound for CTAs of one to three workers, so 128 registers a thread.  The kernels for more
+// than five negatives and d > 128 spill 270 to 370 bytes of them, all others at most 108.
 template <int S, int OM, int DFIX, int NC>
 __global__ void __launch_bounds__(32 * (kCompute + 1) * kTeamMaxPerCta) team_engine_kernel(TrainParams p) {
   extern __shared__ __align__(16) float smem[];

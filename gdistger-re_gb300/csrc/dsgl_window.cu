@@ -11,17 +11,19 @@
 //     written back (stochastically rounded for bf16 tables) when it leaves it,
 //   * the step's output rows (target of each walk + shared negatives) and gradients;
 // the window bookkeeping (vertex and count of each slot, slot of each position) lives in
-// registers, one slot per lane.  dsgl_team.cuh trains a worker with five warps instead; this
-// kernel is the faster one where workers fill the GPU (from about six per SM).
+// registers, one slot per lane.  dsgl_team.cuh trains a worker with five warps instead, the
+// faster way while an SM gets no more than the three teams it holds; of this kernel's workers
+// it holds seven (d = 128, w = 10).
 // Negative rows are read from and added to Woh at each step, as the reference does for
 // the two target rows (dsgl.hpp:1346-1356).  Dot products of the forward are summed as
 // eight sequential partial sums (even and odd k of each quarter of [0, d)) combined
 // pairwise, in register tiles (forward_tiled); the backward keeps the reference's order.
 // What bounds it: the dependent instruction stream of each worker at seven warps per SM
-// (shared memory 30 KB and about 240 registers per thread), then the 128 bytes per cycle that
-// shared memory returns to the registers.  The register tiles read a third of the bytes that
-// one lane per input did, and the gradients are kept once instead of as pairs: 1.1M vertices,
-// 1064 workers, d = 128: bf16 182.3 -> 159.7 ms a pass, d = 64 21.2 -> 16.7 (400k vertices).
+// (shared memory 30 KB and about 240 registers per thread; 34% of the issue slots used), then
+// the 128 bytes per cycle that shared memory returns to the registers (40% of them used).  The
+// register tiles read a third of the bytes that one lane per input did, and the gradients are
+// kept once instead of as pairs: 1.1M vertices, 1064 workers, d = 128: bf16 182.3 -> 159.3 ms a
+// pass, d = 64 21.2 -> 16.7 (400k vertices).
 // Table rows are read past the L1 (load_l2): a line there can be older than what another SM's
 // worker has stored, and would be written back as it was (100k vertices, 250 workers: AUC
 // 0.7764 -> 0.7770 in bf16, 0.7779 -> 0.7786 in fp32; pass times are the same).
