@@ -429,7 +429,30 @@ __global__ void __launch_bounds__(256) validate_csr_kernel(const int64_t* __rest
   }
 }
 
+// Offsets that a caller brings, before any walk is written at them: the first is 0 and each
+// walk takes 1 to max_length vertices and its -1.  got[0]: 1 if not so, got[1]: the last
+// offset (2M walks: 16 MB read, 6 us).
+__global__ void __launch_bounds__(256) validate_offsets_kernel(const int64_t* __restrict__ offsets, int64_t n,
+                                                               int max_length, int64_t* got) {
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < n; w += stride) {
+    const int64_t x = offsets[w], next = offsets[w + 1];
+    const uint64_t vertices = (uint64_t)next - (uint64_t)x - 1;
+    if ((w == 0 && x != 0) || vertices - 1 >= (uint64_t)max_length) got[0] = 1;
+    if (w == n - 1) got[1] = next;
+  }
+}
+
 }  // namespace
+
+cudaError_t launch_validate_offsets(const int64_t* offsets, int64_t walker_num, int max_length, int64_t* got,
+                                    int num_sms, cudaStream_t s) {
+  cudaError_t e = cudaMemsetAsync(got, 0, 2 * sizeof(int64_t), s);
+  if (e != cudaSuccess) return e;
+  const int64_t want = (walker_num + 255) / 256, cap = (int64_t)num_sms * 16;
+  validate_offsets_kernel<<<(unsigned)(want < cap ? want : cap), 256, 0, s>>>(offsets, walker_num, max_length, got);
+  return cudaGetLastError();
+}
 
 cudaError_t launch_validate_csr(const int64_t* indptr, const int32_t* indices, int64_t V, int64_t E,
                                 int32_t* status, int num_sms, cudaStream_t s) {

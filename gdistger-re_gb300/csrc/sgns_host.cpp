@@ -1670,13 +1670,25 @@ struct WalkCall {
                                      o->max_length, o->r_threshold, o->seed, o->trace_steps, at(256 + kTables), sms,
                                      offsets, s)) != cudaSuccess)
       return fail(nullptr, SGNS_ECUDA, "walks: %s", cudaGetErrorString(e));
-    return read_total(offsets, total);
-  }
-  sgns_status read_total(const int64_t* offsets, int64_t* total) {
-    cudaError_t e;
     if ((e = cudaMemcpyAsync(total, offsets + o->walker_num, sizeof *total, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
         (e = cudaStreamSynchronize(s)) != cudaSuccess)
       return fail(nullptr, SGNS_ECUDA, "walks: %s", cudaGetErrorString(e));
+    return SGNS_OK;
+  }
+  // the graph and a caller's offsets, which the walks are written at
+  sgns_status check(const int64_t* offsets, int64_t* total) {
+    sgns_status st = ds->ensure(64);
+    if (st) return st;
+    if ((st = check_csr("walks", indptr, indices, V, n_edges, reinterpret_cast<int32_t*>(at(0)), sms, s))) return st;
+    int64_t* got = reinterpret_cast<int64_t*>(at(16));
+    int64_t h[2] = {0, 0};
+    cudaError_t e;
+    if ((e = launch_validate_offsets(offsets, o->walker_num, o->max_length, got, sms, s)) != cudaSuccess ||
+        (e = cudaMemcpyAsync(h, got, sizeof h, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(s)) != cudaSuccess)
+      return fail(nullptr, SGNS_ECUDA, "walks: %s", cudaGetErrorString(e));
+    if (h[0]) return fail(nullptr, SGNS_EINVAL, "walk offsets must start at 0 and leave each walk 1 to %d vertices", o->max_length);
+    *total = h[1];
     return SGNS_OK;
   }
   sgns_status emit(const int64_t* offsets, int32_t* corpus) {
@@ -1742,11 +1754,8 @@ sgns_status sgns_info_walk_tokens(const sgns_walk_options* o, const int64_t* ind
   if (o->walker_num == 0) return SGNS_OK;
   WalkCall c{o, indptr, indices, cn, V, n_edges, static_cast<cudaStream_t>(stream), 0, nullptr, {}};
   int64_t total = 0;
-  if ((st = c.open()) || (st = c.ds->ensure(64)) ||
-      (st = check_csr("walks", indptr, indices, V, n_edges, reinterpret_cast<int32_t*>(c.at(0)), c.sms, c.s)) ||
-      (st = c.read_total(offsets, &total)))
-    return st;
-  if (total < 0 || total > cap)
+  if ((st = c.open()) || (st = c.check(offsets, &total))) return st;
+  if (total > cap)
     return fail(nullptr, SGNS_EINVAL, "walks yield %lld tokens, capacity %lld", (long long)total, (long long)cap);
   return c.emit(offsets, corpus);
 }

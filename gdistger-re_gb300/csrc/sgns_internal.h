@@ -234,6 +234,10 @@ cudaError_t launch_link_scores(int storage, const void* table, int d, int64_t V,
 constexpr int kWalkMaxLength = 1000;  // vertices per walk (the trainer's limit, dsgl.hpp:23)
 cudaError_t launch_validate_csr(const int64_t* indptr, const int32_t* indices, int64_t V, int64_t E,
                                 int32_t* status, int num_sms, cudaStream_t s);
+// walk offsets (walker_num + 1 entries): got[0] = 1 if they are not those of walks of 1 to
+// max_length vertices, got[1] = the last one (device memory)
+cudaError_t launch_validate_offsets(const int64_t* offsets, int64_t walker_num, int max_length, int64_t* got,
+                                    int num_sms, cudaStream_t s);
 cudaError_t launch_edge_common_neighbors(const int64_t* indptr, const int32_t* indices, int64_t V, int64_t E,
                                          int32_t* cn, int32_t* status, int num_sms, cudaStream_t s);
 size_t walk_scratch_bytes(int64_t walker_num);

@@ -303,7 +303,8 @@ sgns_status sgns_info_walks(const sgns_walk_options* opt, const int64_t* indptr,
  * once and the corpus is allocated in between.  offsets: device memory, walker_num + 1
  * entries: walk k's first token and, last, *n_tokens (nothing is written for no walkers).
  * The second call takes the offsets as the first one wrote them for the same options and
- * graph; cap below the last of them: SGNS_EINVAL and nothing written. */
+ * graph.  SGNS_EINVAL and nothing written: cap below the last of them, or offsets that do not
+ * start at 0 or do not leave every walk 1 to max_length vertices and its -1. */
 sgns_status sgns_info_walk_offsets(const sgns_walk_options* opt, const int64_t* indptr, const int32_t* indices,
                                    const int32_t* cn, int64_t V, int64_t n_edges, int64_t* offsets,
                                    int64_t* n_tokens, void* stream);

@@ -103,3 +103,24 @@ def test_walk_tokens_refuse_a_small_corpus(sgns_lib, oracle_mod):
     assert tokens(len(want) - 1) == sgns.EINVAL and bool((corpus == -9).all())
     assert tokens(len(want)) == sgns.OK and np.array_equal(corpus.cpu().numpy(), want)
     assert sgns_lib.sgns_info_walk_offsets(*graph, None, ctypes.byref(n), None) == sgns.EINVAL
+
+
+@pytest.mark.parametrize("at,value", [(0, 3), (0, -1), (1, -4), (1, 0), (250, 1 << 40), (250, -(1 << 62)), (499, 1),
+                                      (500, 7), (500, -1)])
+def test_walk_tokens_refuse_offsets_that_are_not_walks(at, value, sgns_lib, oracle_mod):
+    """The walks are written where the offsets say: any that would lead outside the corpus is
+    refused before the first token."""
+    import ctypes
+
+    import torch
+
+    ip, ix = clique_and_tail(9, 40)
+    dip, dix, dcn = *on_gpu(ip, ix), torch.from_numpy(oracle_mod.edge_common_neighbors(ip, ix)).cuda()
+    o = sgns.WalkOptions(walker_num=500, min_length=5, max_length=40, r_threshold=0.9, seed=11, trace_steps=1)
+    graph = (ctypes.byref(o), dip.data_ptr(), dix.data_ptr(), dcn.data_ptr(), len(ip) - 1, len(ix))
+    offsets, n = torch.empty(501, dtype=torch.int64, device="cuda"), ctypes.c_int64()
+    assert sgns_lib.sgns_info_walk_offsets(*graph, offsets.data_ptr(), ctypes.byref(n), None) == sgns.OK
+    offsets[at] = value
+    corpus = torch.full((n.value,), -9, dtype=torch.int32, device="cuda")
+    assert sgns_lib.sgns_info_walk_tokens(*graph, offsets.data_ptr(), corpus.data_ptr(), n.value, None) == sgns.EINVAL
+    assert bool((corpus == -9).all())
