@@ -370,6 +370,17 @@ def edge_common_neighbors(indptr, indices, cn, stream=0):
                                             cn.data_ptr() if E else None, ctypes.c_void_p(stream)))
 
 
+def _after_current(stream, device):
+    """Work on `stream` (a handle; 0: the default stream) starts after what is queued on torch's
+    current stream: a new tensor's memory may still be in use there."""
+    import torch
+
+    current = torch.cuda.current_stream(device)
+    if current.cuda_stream != stream:
+        s = torch.cuda.ExternalStream(stream, device) if stream else torch.cuda.default_stream(device)
+        s.wait_stream(current)
+
+
 def info_walks(indptr, indices, cn, walker_num, min_length=20, max_length=80, r_threshold=0.999, seed=1,
                corpus=None, stream=0, trace=1):
     """sgns_info_walks on device tensors.  corpus: int32 device tensor to fill (None: a new
@@ -382,6 +393,7 @@ def info_walks(indptr, indices, cn, walker_num, min_length=20, max_length=80, r_
     n = ctypes.c_int64()
     args = (indptr.data_ptr(), indices.data_ptr() if E else None, cn.data_ptr() if E else None, V, E)
     if corpus is None:  # the lengths, then a corpus of their sum
+        _after_current(stream, indptr.device)
         try:
             offsets = torch.empty(max(o.walker_num, 0) + 1, dtype=torch.int64, device=indptr.device)
         except RuntimeError:  # no room for 8 bytes a walk

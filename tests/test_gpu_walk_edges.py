@@ -124,3 +124,27 @@ def test_walk_tokens_refuse_offsets_that_are_not_walks(at, value, sgns_lib, orac
     corpus = torch.full((n.value,), -9, dtype=torch.int32, device="cuda")
     assert sgns_lib.sgns_info_walk_tokens(*graph, offsets.data_ptr(), corpus.data_ptr(), n.value, None) == sgns.EINVAL
     assert bool((corpus == -9).all())
+
+
+def test_walks_from_another_stream_wait_for_their_corpus(sgns_lib):
+    """Torch's current stream still writes the memory that the new corpus gets: the walks, on the
+    default stream, come after that."""
+    import torch
+
+    ip, ix = on_gpu(*clique_and_tail(40, 0))
+    cn = torch.empty(ix.numel(), dtype=torch.int32, device="cuda")
+    sgns.edge_common_neighbors(ip, ix, cn)
+    walks = lambda: sgns.info_walks(ip, ix, cn, 100_000, 20, 60, 0.9, 5)
+    want, n = walks()
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        held = torch.empty(n, dtype=torch.int32, device="cuda")
+        side.synchronize()
+        place = held.data_ptr()
+        torch.cuda._sleep(400_000_000)  # 0.2 s
+        held.fill_(-7)
+        del held
+        got, _ = walks()
+    torch.cuda.synchronize()
+    assert got.data_ptr() == place and torch.equal(got, want)
