@@ -431,7 +431,7 @@ __global__ void __launch_bounds__(256) validate_csr_kernel(const int64_t* __rest
 
 // Offsets that a caller brings, before any walk is written at them: the first is 0 and each
 // walk takes 1 to max_length vertices and its -1.  got[0]: 1 if not so, got[1]: the last
-// offset (2M walks: 16 MB read, 6 us).
+// offset.  8 bytes a walk: no difference in a call of 2M walks (10.4 ms with it and without).
 __global__ void __launch_bounds__(256) validate_offsets_kernel(const int64_t* __restrict__ offsets, int64_t n,
                                                                int max_length, int64_t* got) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
