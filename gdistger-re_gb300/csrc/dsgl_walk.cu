@@ -46,6 +46,7 @@
 // is needed.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "sgns_internal.h"
@@ -336,12 +337,15 @@ __global__ void add_tile_offsets_kernel(int64_t* offsets, int64_t n, const int64
 }
 
 // ---- common-neighbour counts ----------------------------------------------------------
-// One thread per directed edge e = (u, v).  A block takes tiles of consecutive edges: the
-// sources of a tile's first and last edge are found in indptr once, every other source between
-// them.  The entries of the shorter adjacency list are searched in the longer one: by the
-// thread itself up to kOwnEntries of them, else by the whole warp, edge after edge.
-// status bits: 1 = a neighbour outside [0, V), 2 = an adjacency list not strictly increasing.
-constexpr int kEdgeTile = 256, kOwnEntries = 24;
+// The entries of an edge's shorter adjacency list are searched in the longer one: up to
+// `own` of them by one thread (edge_cn_kernel), else by a warp (edge_cn_long_kernel).  The
+// long lists are those of edges between hubs, which follow one another (a hub's edges are
+// consecutive, and its neighbours begin with the other hubs where ids follow degree), so the
+// second kernel spreads them over the GPU.  What bounds them: the searches' dependent loads.  A
+// power law's (gamma 2.1, ids by degree) 2.2M vertices and 32M edges, and 20k and 321k: 81 and
+// 0.77 ms a call with the long lists left to the warps that came to them, 77 and 0.33 with a warp
+// for every edge, 44 and 0.26 now.  1.1M vertices and 6.3M edges without hubs: 0.40, 4.2, 0.33.
+constexpr int kEdgeWarps = 8, kEdgeThreads = 32 * kEdgeWarps, kOwnEntries = 24;
 
 // the largest u in [lo, hi) with indptr[u] <= e
 __device__ __forceinline__ int64_t source_of(const int64_t* __restrict__ indptr, int64_t e, int64_t lo, int64_t hi) {
@@ -352,62 +356,96 @@ __device__ __forceinline__ int64_t source_of(const int64_t* __restrict__ indptr,
   }
   return lo;
 }
-// entries [i, se) by `step` of the shorter list that the sorted list [lb, le) holds
-__device__ __forceinline__ int count_in(const int32_t* __restrict__ indices, int64_t i, int64_t se, int step, int64_t lb,
-                                        int64_t le) {
-  int c = 0;
-  for (; i < se; i += step) {
-    const int32_t x = __ldg(&indices[i]);
-    int64_t l = lb, h = le;  // first position with indices >= x
-    while (l < h) {
-      const int64_t m = (l + h) >> 1;
-      if (__ldg(&indices[m]) < x) l = m + 1;
-      else h = m;
-    }
-    c += (l < le && __ldg(&indices[l]) == x);
+// 1 when the sorted list of n >= 1 entries holds x.  Lists of one length take the same steps
+// whatever x is, so the lanes of a warp that search one list stay together.
+__device__ __forceinline__ int holds(const int32_t* __restrict__ list, int n, int32_t x) {
+  while (n > 1) {  // the last entry <= x, if any, is one of list[0..n)
+    const int h = n >> 1;
+    list += __ldg(list + h) <= x ? h : 0;
+    n -= h;
   }
-  return c;
+  return __ldg(list) == x;
 }
-__global__ void __launch_bounds__(kEdgeTile) edge_cn_kernel(const int64_t* __restrict__ indptr,
-                                                            const int32_t* __restrict__ indices, int64_t V, int64_t E,
-                                                            int32_t* __restrict__ cn, int32_t* status) {
-  __shared__ int64_t range[2];
+// An edge's two lists, the shorter one first
+struct EdgeLists {
+  const int32_t *s, *l;
+  int ns, nl;
+  __device__ __forceinline__ EdgeLists(const int64_t* __restrict__ indptr, const int32_t* __restrict__ indices, int64_t u,
+                                       int32_t v) {
+    const int64_t ub = __ldg(&indptr[u]), vb = __ldg(&indptr[v]);
+    const int nu = (int)(__ldg(&indptr[u + 1]) - ub), nv = (int)(__ldg(&indptr[(int64_t)v + 1]) - vb);
+    const bool u_short = nu <= nv;
+    s = indices + (u_short ? ub : vb), l = indices + (u_short ? vb : ub);
+    ns = u_short ? nu : nv, nl = u_short ? nv : nu;
+  }
+};
+
+// One thread per directed edge e = (u, v), 32 consecutive ones to a warp: the sources of the
+// first and the last are found in indptr, every other source between them.  cn[e]: the count,
+// or ~u for an edge left to edge_cn_long_kernel.
+// status bits: 1 = a neighbour outside [0, V), 2 = an adjacency list not strictly increasing.
+__global__ void __launch_bounds__(kEdgeThreads) edge_cn_kernel(const int64_t* __restrict__ indptr,
+                                                               const int32_t* __restrict__ indices, int64_t V, int64_t E,
+                                                               int own, int32_t* __restrict__ cn, int32_t* status) {
   const int lane = threadIdx.x & 31;
-  for (int64_t base = (int64_t)blockIdx.x * kEdgeTile; base < E; base += (int64_t)gridDim.x * kEdgeTile) {
-    __syncthreads();
-    if (threadIdx.x < 2) {
-      const int64_t last = base + kEdgeTile < E ? base + kEdgeTile - 1 : E - 1;
-      range[threadIdx.x] = source_of(indptr, threadIdx.x ? last : base, 0, V);
-    }
-    __syncthreads();
-    const int64_t e = base + threadIdx.x;
-    int64_t sb = 0, se = 0, lb = 0, le = 0;
+  const int64_t stride = (int64_t)gridDim.x * kEdgeThreads;
+  for (int64_t base = (int64_t)blockIdx.x * kEdgeThreads + threadIdx.x - lane; base < E; base += stride) {
+    int64_t u = 0;
+    if (lane < 2) u = source_of(indptr, lane == 0 ? base : base + 32 < E ? base + 31 : E - 1, 0, V);
+    const int64_t u0 = __shfl_sync(0xFFFFFFFFu, u, 0), u1 = __shfl_sync(0xFFFFFFFFu, u, 1);
+    const int64_t e = base + lane;
     if (e < E) {
-      const int64_t u = source_of(indptr, e, range[0], range[1] + 1);
+      u = source_of(indptr, e, u0, u1 + 1);
       const int32_t v = __ldg(&indices[e]);
+      int c = 0;
       if (v < 0 || v >= V) {
         atomicOr(status, 1);
       } else {
-        const int64_t ub = __ldg(&indptr[u]), ue = __ldg(&indptr[u + 1]);
-        if (e > ub && __ldg(&indices[e - 1]) >= v) atomicOr(status, 2);
-        const int64_t vb = __ldg(&indptr[v]), ve = __ldg(&indptr[v + 1]);
-        const bool u_short = ue - ub <= ve - vb;
-        sb = u_short ? ub : vb, se = u_short ? ue : ve;
-        lb = u_short ? vb : ub, le = u_short ? ve : ue;
+        if (e > __ldg(&indptr[u]) && __ldg(&indices[e - 1]) >= v) atomicOr(status, 2);
+        const EdgeLists a(indptr, indices, u, v);
+        if (a.ns > own) c = ~(int32_t)u;
+        else
+          for (int i = 0; i < a.ns; i++) c += holds(a.l, a.nl, __ldg(a.s + i));
       }
+      cn[e] = c;
     }
-    const bool own = se - sb <= kOwnEntries;
-    int c = own ? count_in(indices, sb, se, 1, lb, le) : 0;
-    unsigned rest = __ballot_sync(0xFFFFFFFFu, !own);
-    while (rest) {
-      const int k = __ffs(rest) - 1;
-      rest &= rest - 1;
-      const int64_t b = __shfl_sync(0xFFFFFFFFu, sb, k), n = __shfl_sync(0xFFFFFFFFu, se, k);
-      const int64_t l0 = __shfl_sync(0xFFFFFFFFu, lb, k), l1 = __shfl_sync(0xFFFFFFFFu, le, k);
-      const int t = __reduce_add_sync(0xFFFFFFFFu, count_in(indices, b + lane, n, 32, l0, l1));
-      if (lane == k) c = t;
+  }
+}
+
+// The edges left by edge_cn_kernel.  A block looks through eight runs of `run` edges, one per
+// warp, that lie evenly over all edges, and its warps take what is left of them in turn.
+__global__ void __launch_bounds__(kEdgeThreads) edge_cn_long_kernel(const int64_t* __restrict__ indptr,
+                                                                    const int32_t* __restrict__ indices, int64_t E,
+                                                                    int run, int32_t* cn) {
+  __shared__ int64_t queue_e[kEdgeThreads];
+  __shared__ int32_t queue_u[kEdgeThreads];
+  __shared__ int queued, taken;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t runs = (E + run - 1) / run;
+  if (threadIdx.x == 0) queued = taken = 0;
+  for (int64_t first = blockIdx.x; first < runs; first += kEdgeWarps * (int64_t)gridDim.x) {
+    const int64_t e = (first + warp * (int64_t)gridDim.x) * run + lane;
+    const int32_t left = lane < run && e < E ? cn[e] : 0;
+    if (!__syncthreads_or(left < 0)) continue;
+    if (left < 0) {
+      const int k = atomicAdd(&queued, 1);
+      queue_e[k] = e;
+      queue_u[k] = ~left;
     }
-    if (e < E) cn[e] = c;
+    __syncthreads();
+    while (true) {
+      int k = 0;
+      if (lane == 0) k = atomicAdd(&taken, 1);
+      k = __shfl_sync(0xFFFFFFFFu, k, 0);
+      if (k >= queued) break;
+      const EdgeLists a(indptr, indices, queue_u[k], __ldg(&indices[queue_e[k]]));
+      int c = 0;
+      for (int i = lane; i - lane < a.ns; i += 32) c += i < a.ns ? holds(a.l, a.nl, __ldg(a.s + i)) : 0;
+      c = __reduce_add_sync(0xFFFFFFFFu, c);
+      if (lane == 0) cn[queue_e[k]] = c;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) queued = taken = 0;  // before the next round's first barrier
   }
 }
 
@@ -529,9 +567,18 @@ cudaError_t launch_info_walks_emit(const int64_t* indptr, const int32_t* indices
 cudaError_t launch_edge_common_neighbors(const int64_t* indptr, const int32_t* indices, int64_t V, int64_t E,
                                          int32_t* cn, int32_t* status, int num_sms, cudaStream_t s) {
   if (E == 0) return cudaSuccess;
-  const int64_t want = (E + kEdgeTile - 1) / kEdgeTile;
-  const int64_t cap = (int64_t)num_sms * 64;
-  edge_cn_kernel<<<(unsigned)(want < cap ? want : cap), kEdgeTile, 0, s>>>(indptr, indices, V, E, cn, status);
+  const int64_t want = (E + kEdgeThreads - 1) / kEdgeThreads, cap = (int64_t)num_sms * 64;
+  const int64_t warps = (int64_t)num_sms * 8 * kEdgeWarps;  // eight blocks per SM
+  // Up to four edges per warp of the GPU (39k) a thread's own chain of searches is the call:
+  // nearly all go to a warp (2,000 vertices of a power law, 31k edges: 81 -> 65 us; above, at 114k
+  // edges of a flat graph, 53 -> 77).
+  const int own = E <= 4 * warps ? 2 : kOwnEntries;
+  edge_cn_kernel<<<(unsigned)std::min(want, cap), kEdgeThreads, 0, s>>>(indptr, indices, V, E, own, cn, status);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  const int run = (int)std::min<int64_t>(32, (E + warps - 1) / warps);
+  const int64_t blocks = (E + (int64_t)run * kEdgeWarps - 1) / ((int64_t)run * kEdgeWarps);
+  edge_cn_long_kernel<<<(unsigned)std::min(blocks, cap), kEdgeThreads, 0, s>>>(indptr, indices, E, run, cn);
   return cudaGetLastError();
 }
 

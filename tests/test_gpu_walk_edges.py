@@ -148,3 +148,49 @@ def test_walks_from_another_stream_wait_for_their_corpus(sgns_lib):
         got, _ = walks()
     torch.cuda.synchronize()
     assert got.data_ptr() == place and torch.equal(got, want)
+
+
+@pytest.mark.parametrize("past", [0, 1])
+def test_common_neighbors_around_the_small_graphs(past, sgns_lib, oracle_mod):
+    """Up to 4 x 64 edges per SM lists of three entries go to a warp, above those of 25."""
+    import torch
+
+    edges = 256 * torch.cuda.get_device_properties(0).multi_processor_count + 2 * past
+    ip, ix = clique_and_tail(30, (edges - 30 * 29) // 2)
+    assert len(ix) == edges
+    cn = torch.empty(edges, dtype=torch.int32, device="cuda")
+    sgns.edge_common_neighbors(*on_gpu(ip, ix), cn)
+    assert np.array_equal(cn.cpu().numpy(), oracle_mod.edge_common_neighbors(ip, ix))
+
+
+def test_common_neighbors_take_as_long_in_any_order_of_the_vertices(sgns_lib, oracle_mod):
+    """The same power-law graph with its ids by degree and shuffled: the same searches, so about
+    the same time, though by degree the hubs' edges follow one another (1.5 is far above the
+    scatter of a median; hubs' edges on a few SMs take several times as long)."""
+    import torch
+
+    import synth
+
+    V = 20_000
+    ip, ix = synth.chung_lu(V, 54_600, 2.1, seed=3, device="cuda")
+    src = torch.repeat_interleave(torch.arange(V, device="cuda"), ip.diff())
+    new = torch.randperm(V, generator=torch.Generator().manual_seed(1)).cuda()
+    key, order = torch.sort(new[src] * V + new[ix.long()])
+    sip = torch.searchsorted(torch.div(key, V, rounding_mode="floor"), torch.arange(V + 1, device="cuda"))
+    six = (key % V).to(torch.int32)
+    counts, medians = [], []
+    for p, x in ((ip, ix), (sip, six)):
+        cn = torch.empty_like(x)
+        times = []
+        for _ in range(15):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            sgns.edge_common_neighbors(p, x, cn)
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        counts.append(cn)
+        medians.append(sorted(times)[len(times) // 2])
+    assert np.array_equal(counts[0].cpu().numpy(), oracle_mod.edge_common_neighbors(ip.cpu().numpy(), ix.cpu().numpy()))
+    assert torch.equal(counts[0][order], counts[1])
+    assert medians[0] < 1.5 * medians[1], medians
