@@ -106,6 +106,7 @@ struct WalkArgs {
   double r_threshold;
   uint64_t seed;
   int32_t trace;           // 1: the trace step of walk.hpp:920-1031; 0: moves only
+  const int32_t* refused;  // not 0: an input was refused, nothing is walked
   int32_t* lengths;        // pass 1 output
   const int64_t* offsets;  // pass 2 input (exclusive scan of length + 1)
   int32_t* corpus;         // pass 2 output
@@ -192,6 +193,7 @@ struct Walker {
 // histories, four vertices to an int4, [ceil(max_length / 4)][blockDim.x].
 __global__ void __launch_bounds__(256) walk_lengths_kernel(WalkArgs a) {
   extern __shared__ __align__(16) unsigned char walk_smem[];
+  if (*a.refused) return;
   const int T = blockDim.x, tid = threadIdx.x, entries = a.max_length + 2;
   LengthTable* tab = reinterpret_cast<LengthTable*>(walk_smem);
   double* xl = reinterpret_cast<double*>(tab + entries);
@@ -247,6 +249,7 @@ __global__ void __launch_bounds__(256) walk_lengths_kernel(WalkArgs a) {
 
 // Pass 2: the walk's tokens and its -1 at offsets[w].
 __global__ void __launch_bounds__(256) walk_tokens_kernel(WalkArgs a) {
+  if (*a.refused) return;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   Walker k{};
@@ -330,10 +333,11 @@ __global__ void __launch_bounds__(kScanBlock) scan_tile_sums_kernel(int64_t* til
   if (threadIdx.x == 0) tile_sums[n_tiles] = carry;
 }
 
-__global__ void add_tile_offsets_kernel(int64_t* offsets, int64_t n, const int64_t* tile_sums, int64_t n_tiles) {
+__global__ void add_tile_offsets_kernel(int64_t* offsets, int64_t n, const int64_t* tile_sums, int64_t n_tiles,
+                                        WalkReport* report) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) offsets[i] += tile_sums[i / kScanBlock];
-  if (i == 0) offsets[n] = tile_sums[n_tiles];
+  if (i == 0) offsets[n] = report->total = tile_sums[n_tiles];
 }
 
 // ---- common-neighbour counts ----------------------------------------------------------
@@ -467,28 +471,31 @@ __global__ void __launch_bounds__(256) validate_csr_kernel(const int64_t* __rest
   }
 }
 
-// Offsets that a caller brings, before any walk is written at them: the first is 0 and each
-// walk takes 1 to max_length vertices and its -1.  got[0]: 1 if not so, got[1]: the last
-// offset.  8 bytes a walk: no difference in a call of 2M walks (10.4 ms with it and without).
+// Offsets that a caller brings, before any walk is written at them.  report: total, the last
+// offset; refused bits: 8 = the first is not 0 or a walk has not 1 to max_length vertices and its
+// -1, 16 = the last is above cap.  8 bytes a walk: no difference in a call of 2M walks (10.4 ms
+// with it and without).
 __global__ void __launch_bounds__(256) validate_offsets_kernel(const int64_t* __restrict__ offsets, int64_t n,
-                                                               int max_length, int64_t* got) {
+                                                               int max_length, int64_t cap, WalkReport* report) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < n; w += stride) {
     const int64_t x = offsets[w], next = offsets[w + 1];
     const uint64_t vertices = (uint64_t)next - (uint64_t)x - 1;
-    if ((w == 0 && x != 0) || vertices - 1 >= (uint64_t)max_length) got[0] = 1;
-    if (w == n - 1) got[1] = next;
+    if ((w == 0 && x != 0) || vertices - 1 >= (uint64_t)max_length) atomicOr(&report->refused, 8);
+    if (w == n - 1) {
+      report->total = next;
+      if (next > cap) atomicOr(&report->refused, 16);
+    }
   }
 }
 
 }  // namespace
 
-cudaError_t launch_validate_offsets(const int64_t* offsets, int64_t walker_num, int max_length, int64_t* got,
-                                    int num_sms, cudaStream_t s) {
-  cudaError_t e = cudaMemsetAsync(got, 0, 2 * sizeof(int64_t), s);
-  if (e != cudaSuccess) return e;
-  const int64_t want = (walker_num + 255) / 256, cap = (int64_t)num_sms * 16;
-  validate_offsets_kernel<<<(unsigned)(want < cap ? want : cap), 256, 0, s>>>(offsets, walker_num, max_length, got);
+cudaError_t launch_validate_offsets(const int64_t* offsets, int64_t walker_num, int max_length, int64_t cap,
+                                    WalkReport* report, int num_sms, cudaStream_t s) {
+  const int64_t want = (walker_num + 255) / 256, most = (int64_t)num_sms * 16;
+  validate_offsets_kernel<<<(unsigned)(want < most ? want : most), 256, 0, s>>>(offsets, walker_num, max_length, cap,
+                                                                                report);
   return cudaGetLastError();
 }
 
@@ -525,16 +532,17 @@ size_t walk_scratch_bytes(int64_t walker_num) {
   return sizeof(int32_t) * (size_t)walker_num + sizeof(int64_t) * (size_t)(tiles + 1);
 }
 
-// Pass 1 (lengths) and the scan: offsets, walker_num + 1 entries, the last = total tokens.
+// Pass 1 (lengths) and the scan: offsets, walker_num + 1 entries, the last = total tokens (also
+// in the report).
 cudaError_t launch_info_walks_count(const int64_t* indptr, const int32_t* indices, const int32_t* cn,
                                     const double* xl, const double* len_table, int64_t V, int64_t walker_num,
                                     int min_length, int max_length, double r_threshold, uint64_t seed, int trace,
-                                    void* scratch, int num_sms, int64_t* offsets, cudaStream_t s) {
+                                    void* scratch, int num_sms, int64_t* offsets, WalkReport* report, cudaStream_t s) {
   const int64_t tiles = (walker_num + kScanBlock - 1) / kScanBlock;
   int64_t* tile_sums = static_cast<int64_t*>(scratch);
   int32_t* lengths = reinterpret_cast<int32_t*>(tile_sums + tiles + 1);
   const WalkArgs a{indptr, indices, cn, xl, reinterpret_cast<const LengthTable*>(len_table), V, walker_num, min_length,
-                   max_length, r_threshold, seed, trace, lengths, nullptr, nullptr};
+                   max_length, r_threshold, seed, trace, &report->refused, lengths, nullptr, nullptr};
   const int T = walk_block_threads(max_length);
   const size_t smem = walk_smem(max_length, T);
   cudaError_t e = cudaFuncSetAttribute(walk_lengths_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -548,17 +556,18 @@ cudaError_t launch_info_walks_count(const int64_t* indptr, const int32_t* indice
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   scan_tiles_kernel<<<(unsigned)tiles, kScanBlock, 0, s>>>(lengths, walker_num, offsets, tile_sums);
   scan_tile_sums_kernel<<<1, kScanBlock, 0, s>>>(tile_sums, tiles);
-  add_tile_offsets_kernel<<<(unsigned)((walker_num + 256) / 256), 256, 0, s>>>(offsets, walker_num, tile_sums, tiles);
+  add_tile_offsets_kernel<<<(unsigned)((walker_num + 256) / 256), 256, 0, s>>>(offsets, walker_num, tile_sums, tiles,
+                                                                              report);
   return cudaGetLastError();
 }
 
 // Pass 2: the walks again, written at their offsets.
 cudaError_t launch_info_walks_emit(const int64_t* indptr, const int32_t* indices, const int32_t* cn, int64_t V,
                                    int64_t walker_num, uint64_t seed, int trace, const int64_t* offsets,
-                                   int32_t* corpus, int num_sms, cudaStream_t s) {
+                                   int32_t* corpus, const WalkReport* report, int num_sms, cudaStream_t s) {
   WalkArgs a{};
   a.indptr = indptr, a.indices = indices, a.cn = cn, a.V = V, a.walker_num = walker_num;
-  a.seed = seed, a.trace = trace, a.offsets = offsets, a.corpus = corpus;
+  a.seed = seed, a.trace = trace, a.refused = &report->refused, a.offsets = offsets, a.corpus = corpus;
   const int64_t want = (walker_num + 255) / 256, resident = (int64_t)num_sms * 8;
   walk_tokens_kernel<<<(unsigned)(want < resident ? want : resident), 256, 0, s>>>(a);
   return cudaGetLastError();

@@ -1568,6 +1568,14 @@ sgns_status sgns_link_scores(int32_t dtype, int32_t d, const void* table, int64_
 }
 
 namespace {
+// launch_validate_csr's status word
+sgns_status csr_refused(const char* what, int32_t status, int64_t V) {
+  if (status & 4)
+    return fail(nullptr, SGNS_EINVAL, "%s: indptr must start at 0, end at n_edges and not decrease", what);
+  if (status & 1) return fail(nullptr, SGNS_EINVAL, "%s: a neighbour id lies outside [0, %lld)", what, (long long)V);
+  return SGNS_OK;
+}
+
 // Checks a device CSR graph; status word in scratch.  Returns SGNS_OK or the error.
 sgns_status check_csr(const char* what, const int64_t* indptr, const int32_t* indices, int64_t V, int64_t E,
                       int32_t* status, int sms, cudaStream_t s) {
@@ -1578,9 +1586,7 @@ sgns_status check_csr(const char* what, const int64_t* indptr, const int32_t* in
       (e = cudaMemcpyAsync(&hs, status, sizeof hs, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
       (e = cudaStreamSynchronize(s)) != cudaSuccess)
     return fail(nullptr, SGNS_ECUDA, "%s: %s", what, cudaGetErrorString(e));
-  if (hs & 4) return fail(nullptr, SGNS_EINVAL, "%s: indptr must start at 0, end at n_edges and not decrease", what);
-  if (hs & 1) return fail(nullptr, SGNS_EINVAL, "%s: a neighbour id lies outside [0, %lld)", what, (long long)V);
-  return SGNS_OK;
+  return csr_refused(what, hs, V);
 }
 
 int device_sms() {
@@ -1644,8 +1650,8 @@ struct WalkCall {
     lock = std::unique_lock<std::mutex>(ds->mx);
     return SGNS_OK;
   }
-  // Scratch: a status word, x log2 x, the per-length constants of the update, the length
-  // pass's own, then (own_offsets) the offsets where the caller brings none.
+  // Scratch: the report, x log2 x, the per-length constants of the update, the length pass's
+  // own, then (own_offsets) the offsets where the caller brings none.
   static constexpr int kEntries = kWalkMaxLength + 2;
   static constexpr size_t kTables = sizeof(double) * (size_t)kEntries * (1 + kWalkTableDoubles);
   size_t offsets_at() const { return (256 + kTables + walk_scratch_bytes(o->walker_num) + 7) & ~(size_t)7; }
@@ -1653,51 +1659,44 @@ struct WalkCall {
     return offsets_at() + (own_offsets ? sizeof(int64_t) * (size_t)(o->walker_num + 1) : 0);
   }
   char* at(size_t off) const { return static_cast<char*>(ds->buf) + off; }
+  WalkReport* report() const { return reinterpret_cast<WalkReport*>(at(0)); }
 
+  // the graph checked into a cleared report
+  cudaError_t check_graph() {
+    const cudaError_t e = cudaMemsetAsync(report(), 0, sizeof(WalkReport), s);
+    return e != cudaSuccess ? e : launch_validate_csr(indptr, indices, V, n_edges, &report()->refused, sms, s);
+  }
+  // the report, once the work queued so far is done; e: an error before that
+  sgns_status read(cudaError_t e, WalkReport* r) {
+    if (e != cudaSuccess ||
+        (e = cudaMemcpyAsync(r, report(), sizeof *r, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(s)) != cudaSuccess)
+      return fail(nullptr, SGNS_ECUDA, "walks: %s", cudaGetErrorString(e));
+    return csr_refused("walks", r->refused, V);
+  }
   // the walks' lengths, scanned into offsets (null: the scratch's own)
   sgns_status count(int64_t*& offsets, int64_t* total) {
     sgns_status st = ds->ensure(bytes(!offsets));
     if (st) return st;
     if (!offsets) offsets = reinterpret_cast<int64_t*>(at(offsets_at()));
     double* xl = reinterpret_cast<double*>(at(256));
-    if ((st = check_csr("walks", indptr, indices, V, n_edges, reinterpret_cast<int32_t*>(at(0)), sms, s))) return st;
     std::vector<double> tables(kTables / sizeof(double));
     xlog2x_table(kEntries, tables.data());
     walk_length_table(kEntries, tables.data(), tables.data() + kEntries);
-    cudaError_t e;
-    if ((e = cudaMemcpyAsync(xl, tables.data(), kTables, cudaMemcpyHostToDevice, s)) != cudaSuccess ||
-        (e = launch_info_walks_count(indptr, indices, cn, xl, xl + kEntries, V, o->walker_num, o->min_length,
-                                     o->max_length, o->r_threshold, o->seed, o->trace_steps, at(256 + kTables), sms,
-                                     offsets, s)) != cudaSuccess)
-      return fail(nullptr, SGNS_ECUDA, "walks: %s", cudaGetErrorString(e));
-    if ((e = cudaMemcpyAsync(total, offsets + o->walker_num, sizeof *total, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
-        (e = cudaStreamSynchronize(s)) != cudaSuccess)
-      return fail(nullptr, SGNS_ECUDA, "walks: %s", cudaGetErrorString(e));
+    cudaError_t e = check_graph();
+    if (e == cudaSuccess) e = cudaMemcpyAsync(xl, tables.data(), kTables, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess)
+      e = launch_info_walks_count(indptr, indices, cn, xl, xl + kEntries, V, o->walker_num, o->min_length,
+                                  o->max_length, o->r_threshold, o->seed, o->trace_steps, at(256 + kTables), sms,
+                                  offsets, report(), s);
+    WalkReport r{};
+    if ((st = read(e, &r))) return st;
+    *total = r.total;
     return SGNS_OK;
   }
-  // the graph and a caller's offsets, which the walks are written at
-  sgns_status check(const int64_t* offsets, int64_t* total) {
-    sgns_status st = ds->ensure(64);
-    if (st) return st;
-    if ((st = check_csr("walks", indptr, indices, V, n_edges, reinterpret_cast<int32_t*>(at(0)), sms, s))) return st;
-    int64_t* got = reinterpret_cast<int64_t*>(at(16));
-    int64_t h[2] = {0, 0};
-    cudaError_t e;
-    if ((e = launch_validate_offsets(offsets, o->walker_num, o->max_length, got, sms, s)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(h, got, sizeof h, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
-        (e = cudaStreamSynchronize(s)) != cudaSuccess)
-      return fail(nullptr, SGNS_ECUDA, "walks: %s", cudaGetErrorString(e));
-    if (h[0]) return fail(nullptr, SGNS_EINVAL, "walk offsets must start at 0 and leave each walk 1 to %d vertices", o->max_length);
-    *total = h[1];
-    return SGNS_OK;
-  }
-  sgns_status emit(const int64_t* offsets, int32_t* corpus) {
-    cudaError_t e;
-    if ((e = launch_info_walks_emit(indptr, indices, cn, V, o->walker_num, o->seed, o->trace_steps, offsets, corpus,
-                                    sms, s)) != cudaSuccess ||
-        (e = cudaStreamSynchronize(s)) != cudaSuccess)
-      return fail(nullptr, SGNS_ECUDA, "walks: %s", cudaGetErrorString(e));
-    return SGNS_OK;
+  cudaError_t emit(const int64_t* offsets, int32_t* corpus) {
+    return launch_info_walks_emit(indptr, indices, cn, V, o->walker_num, o->seed, o->trace_steps, offsets, corpus,
+                                  report(), sms, s);
   }
 };
 
@@ -1725,7 +1724,9 @@ sgns_status sgns_info_walks(const sgns_walk_options* o, const int64_t* indptr, c
     if (cap == 0 && !corpus) return SGNS_OK;
     return fail(nullptr, SGNS_EINVAL, "walks yield %lld tokens, capacity %lld", (long long)total, (long long)cap);
   }
-  return c.emit(offsets, corpus);
+  cudaError_t e = c.emit(offsets, corpus);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(c.s);
+  return e == cudaSuccess ? SGNS_OK : fail(nullptr, SGNS_ECUDA, "walks: %s", cudaGetErrorString(e));
 }
 
 sgns_status sgns_info_walk_offsets(const sgns_walk_options* o, const int64_t* indptr, const int32_t* indices,
@@ -1753,11 +1754,18 @@ sgns_status sgns_info_walk_tokens(const sgns_walk_options* o, const int64_t* ind
   if (st) return st;
   if (o->walker_num == 0) return SGNS_OK;
   WalkCall c{o, indptr, indices, cn, V, n_edges, static_cast<cudaStream_t>(stream), 0, nullptr, {}};
-  int64_t total = 0;
-  if ((st = c.open()) || (st = c.check(offsets, &total))) return st;
-  if (total > cap)
-    return fail(nullptr, SGNS_EINVAL, "walks yield %lld tokens, capacity %lld", (long long)total, (long long)cap);
-  return c.emit(offsets, corpus);
+  if ((st = c.open()) || (st = c.ds->ensure(sizeof(WalkReport)))) return st;
+  cudaError_t e = c.check_graph();
+  if (e == cudaSuccess)
+    e = launch_validate_offsets(offsets, o->walker_num, o->max_length, cap, c.report(), c.sms, c.s);
+  if (e == cudaSuccess && cap > 0) e = c.emit(offsets, corpus);
+  WalkReport r{};
+  if ((st = c.read(e, &r))) return st;
+  if (r.refused & 8)
+    return fail(nullptr, SGNS_EINVAL, "walk offsets must start at 0 and leave each walk 1 to %d vertices", o->max_length);
+  if (r.refused & 16)
+    return fail(nullptr, SGNS_EINVAL, "walks yield %lld tokens, capacity %lld", (long long)r.total, (long long)cap);
+  return SGNS_OK;
 }
 
 sgns_status sgns_loss_adjoint(int32_t dtype, int32_t d, int64_t V, int32_t n, const int32_t* in_ptr,

@@ -234,10 +234,16 @@ cudaError_t launch_link_scores(int storage, const void* table, int d, int64_t V,
 constexpr int kWalkMaxLength = 1000;  // vertices per walk (the trainer's limit, dsgl.hpp:23)
 cudaError_t launch_validate_csr(const int64_t* indptr, const int32_t* indices, int64_t V, int64_t E,
                                 int32_t* status, int num_sms, cudaStream_t s);
-// walk offsets (walker_num + 1 entries): got[0] = 1 if they are not those of walks of 1 to
-// max_length vertices, got[1] = the last one (device memory)
-cudaError_t launch_validate_offsets(const int64_t* offsets, int64_t walker_num, int max_length, int64_t* got,
-                                    int num_sms, cudaStream_t s);
+// What a walk call reads back (device memory): bits of the inputs refused, 0 if the walks were
+// made (1 and 4 as launch_validate_csr's status, 8 and 16 as launch_validate_offsets'), and the
+// tokens of all walks.  The walk kernels make nothing when a bit is set, so the host reads it
+// once, behind them.
+struct WalkReport {
+  int32_t refused, pad;
+  int64_t total;
+};
+cudaError_t launch_validate_offsets(const int64_t* offsets, int64_t walker_num, int max_length, int64_t cap,
+                                    WalkReport* report, int num_sms, cudaStream_t s);
 cudaError_t launch_edge_common_neighbors(const int64_t* indptr, const int32_t* indices, int64_t V, int64_t E,
                                          int32_t* cn, int32_t* status, int num_sms, cudaStream_t s);
 size_t walk_scratch_bytes(int64_t walker_num);
@@ -246,10 +252,10 @@ constexpr int kWalkTableDoubles = 4;
 cudaError_t launch_info_walks_count(const int64_t* indptr, const int32_t* indices, const int32_t* cn,
                                     const double* xl, const double* len_table, int64_t V, int64_t walker_num,
                                     int min_length, int max_length, double r_threshold, uint64_t seed, int trace,
-                                    void* scratch, int num_sms, int64_t* offsets, cudaStream_t s);
+                                    void* scratch, int num_sms, int64_t* offsets, WalkReport* report, cudaStream_t s);
 cudaError_t launch_info_walks_emit(const int64_t* indptr, const int32_t* indices, const int32_t* cn, int64_t V,
                                    int64_t walker_num, uint64_t seed, int trace, const int64_t* offsets,
-                                   int32_t* corpus, int num_sms, cudaStream_t s);
+                                   int32_t* corpus, const WalkReport* report, int num_sms, cudaStream_t s);
 
 void host_exp_table(float* t /* kExpTableSize + 1 */);
 int report_error(int status, const char* fmt, ...);  // sets sgns_last_error(NULL); returns status

@@ -301,7 +301,8 @@ sgns_status sgns_info_walks(const sgns_walk_options* opt, const int64_t* indptr,
 
 /* The same in two calls, for a corpus of unknown size: the pass over the walks' lengths runs
  * once and the corpus is allocated in between.  offsets: device memory, walker_num + 1
- * entries: walk k's first token and, last, *n_tokens (nothing is written for no walkers).
+ * entries: walk k's first token and, last, *n_tokens (nothing is written for no walkers; what a
+ * refused call leaves there is undefined).
  * The second call takes the offsets as the first one wrote them for the same options and
  * graph.  SGNS_EINVAL and nothing written: cap below the last of them, or offsets that do not
  * start at 0 or do not leave every walk 1 to max_length vertices and its -1. */

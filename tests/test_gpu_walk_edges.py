@@ -194,3 +194,32 @@ def test_common_neighbors_take_as_long_in_any_order_of_the_vertices(sgns_lib, or
     assert np.array_equal(counts[0].cpu().numpy(), oracle_mod.edge_common_neighbors(ip.cpu().numpy(), ix.cpu().numpy()))
     assert torch.equal(counts[0][order], counts[1])
     assert medians[0] < 1.5 * medians[1], medians
+
+
+def test_walks_over_a_bad_graph_make_nothing(sgns_lib):
+    """A neighbour outside the graph, and an indptr that leads past the edges: each of the walk
+    calls refuses it and leaves the corpus as it was."""
+    import ctypes
+
+    import torch
+
+    good = clique_and_tail(9, 40)
+    cn = torch.zeros(len(good[1]), dtype=torch.int32, device="cuda")
+    o = sgns.WalkOptions(walker_num=500, min_length=5, max_length=40, r_threshold=0.9, seed=11, trace_steps=0)
+    offsets, n = torch.empty(501, dtype=torch.int64, device="cuda"), ctypes.c_int64()
+    corpus = torch.full((500 * 41,), -9, dtype=torch.int32, device="cuda")
+    graph = lambda ip, ix: (ctypes.byref(o), ip.data_ptr(), ix.data_ptr(), cn.data_ptr(), ip.numel() - 1, ix.numel())
+    whole = on_gpu(*good)
+    assert sgns_lib.sgns_info_walk_offsets(*graph(*whole), offsets.data_ptr(), ctypes.byref(n), None) == sgns.OK
+    far, past = on_gpu(*good), on_gpu(*good)
+    far[1][7] = len(good[0]) - 1
+    past[0][20] = len(good[1]) + 1
+    for g in (far, past):
+        calls = ((sgns_lib.sgns_info_walk_tokens, offsets.data_ptr(), corpus.data_ptr(), corpus.numel(), None),
+                 (sgns_lib.sgns_info_walks, corpus.data_ptr(), corpus.numel(), ctypes.byref(n), None),
+                 (sgns_lib.sgns_info_walk_offsets, torch.empty_like(offsets).data_ptr(), ctypes.byref(n), None))
+        for call, *args in calls:
+            n.value = 5
+            assert call(*graph(*g), *args) == sgns.EINVAL and (n.value == 0 or call == calls[0][0])
+        assert bool((corpus == -9).all())
+    assert sgns_lib.sgns_info_walk_tokens(*graph(*whole), offsets.data_ptr(), corpus.data_ptr(), corpus.numel(), None) == sgns.OK
