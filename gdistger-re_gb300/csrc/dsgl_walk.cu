@@ -473,7 +473,7 @@ __global__ void __launch_bounds__(256) validate_csr_kernel(const int64_t* __rest
 
 // Offsets that a caller brings, before any walk is written at them.  report: total, the last
 // offset; refused bits: 8 = the first is not 0 or a walk has not 1 to max_length vertices and its
-// -1, 16 = the last is above cap.  8 bytes a walk: no difference in a call of 2M walks (10.4 ms
+// -1, 16 = the last is above cap.  8 bytes a walk: no difference in a call of 2M walks (10.3 ms
 // with it and without).
 __global__ void __launch_bounds__(256) validate_offsets_kernel(const int64_t* __restrict__ offsets, int64_t n,
                                                                int max_length, int64_t cap, WalkReport* report) {
